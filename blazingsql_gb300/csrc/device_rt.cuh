@@ -31,6 +31,8 @@ __device__ __forceinline__ u64 gx_mod_ii(u64 a, u64 b) {
   const i64 x = (i64)a, y = (i64)b;
   return (y == 0 || y == -1) ? 0ull : (u64)(x % y);
 }
+// the same for operands known to fit 31 bits and a sign
+__device__ __forceinline__ u64 gx_mod_32(int x, int y) { return (y == 0 || y == -1) ? 0ull : (u64)(i64)(x % y); }
 
 // ---- ROUND scale: correctly rounded 10^d for integral |d| <= 22 -------------
 __constant__ double gx_p10[23] = {1e0, 1e1, 1e2, 1e3, 1e4, 1e5, 1e6, 1e7, 1e8, 1e9, 1e10, 1e11,
@@ -70,6 +72,23 @@ __device__ __forceinline__ i64 gx_civil(i64 days, int part) {
   const i64 m = mp < 10 ? mp + 3 : mp - 9;
   const i64 y = yoe + era * 400 + (m <= 2);
   return part == 0 ? y : (part == 1 ? m : d);
+}
+// The same for a DATE's 32-bit day count: within 2^30 days of the epoch the
+// days are counted from 7400 eras (of 400 years) before it, so every division
+// is unsigned and 32 bits wide.  The general form's nine 64-bit divisions by
+// constants are about 25 instructions each.
+__device__ __forceinline__ i64 gx_civil32(int days, int part) {
+  if ((u32)days + (1u << 30) >= (1u << 31)) return gx_civil((i64)days, part);
+  const u32 z = (u32)days + (719468u + 7400u * 146097u);
+  const u32 era = z / 146097u;
+  const u32 doe = z - era * 146097u;
+  const u32 yoe = (doe - doe / 1460u + doe / 36524u - doe / 146096u) / 365u;
+  const u32 doy = doe - (365u * yoe + yoe / 4u - yoe / 100u);
+  const u32 mp = (5u * doy + 2u) / 153u;
+  const u32 d = doy - (153u * mp + 2u) / 5u + 1u;
+  const u32 m = mp < 10u ? mp + 3u : mp - 9u;
+  const int y = (int)(yoe + era * 400u) - 7400 * 400 + (m <= 2u ? 1 : 0);
+  return part == 0 ? (i64)y : (part == 1 ? (i64)m : (i64)d);
 }
 // EXTRACT on a timestamp count with `per_day` units per day (1 for DAYS).
 // which: 0 year, 1 month, 2 day, 3 iso day-of-week, 4 hour, 5 minute, 6 second

@@ -421,6 +421,196 @@ GXE_FN gxe_u64 gxe_div_small(gxe_u64 a, gxe_i64 k, const gxe_u64* rcp, int n) {
   return k < 0 ? q ^ GXE_SIGN : q;
 }
 
+// ---- division by a divisor whose reciprocal is known ahead ------------------
+// Quotients by a literal or by a small integer need no FP64-pipe instruction
+// at all.  That pipe issues one warp instruction every 16 clocks per SM, so the
+// FMA-unit form above (a multiply and two FMAs, plus the conversions of integer
+// operands) holds it for 48 to 80 clocks per 32 rows, where the form below
+// takes about 30 integer instructions (64 lanes a clock on each of the ALU and
+// IMAD pipes).  gxe_quot is that form: with the divisor's reciprocal rounded
+// down to 64 bits (gxe_recip_floor), one 64 x 64 multiply-high gives the
+// quotient's leading 64 bits, at most 4 units too low; the 11 bits below the
+// significand decide the rounding except within 4 units of the midpoint, where
+// the exact remainder's sign does.  (A quotient of two 53-bit significands is
+// never itself a midpoint.)
+
+// floor(2^116 / mb) for a significand mb in [2^52, 2^53); 2^64 - 1 for 2^52
+GXE_FN gxe_u64 gxe_recip_floor(gxe_u64 mb) {
+  // restoring long division: 2^63 / (mb / 2^53) bit by bit
+  gxe_u64 rem = GXE_HIDDEN, q = 0;  // rem < mb unless mb == 2^52
+  if (mb == GXE_HIDDEN) return ~0ull;
+  for (int i = 0; i < 64; i++) {
+    rem <<= 1;
+    q <<= 1;
+    if (rem >= mb) {
+      rem -= mb;
+      q |= 1ull;
+    }
+  }
+  return q;
+}
+
+// A / (mb 2^11) for a normalised numerator A (top bit set, at most 53 leading
+// bits used), r = gxe_recip_floor(mb); e is the quotient's biased exponent when
+// A >= mb 2^11, and [e - 1, e] lies within the normal range (a carry out of
+// the top exponent gives the infinity).
+GXE_FN gxe_u64 gxe_quot(gxe_u64 sign, int e, gxe_u64 A, gxe_u64 mb, gxe_u64 r) {
+  gxe_u64 h = gxe_umulhi(A, r);
+  const int s = (gxe_i64)h < 0 ? 0 : 1;
+  h <<= s;
+  const gxe_u64 m = h >> 11;
+  const unsigned low = (unsigned)h & 0x7FFu;
+  unsigned up = low >> 10;
+  if (low - 0x3FCu < 4u) up = (gxe_i64)((A << (42 + s)) - (2ull * m + 1ull) * mb) > 0 ? 1u : 0u;
+  return sign | (((gxe_u64)(unsigned)(e - 1 - s) << 52) + m + up);
+}
+
+// x / y for the operands no fast path takes (subnormal, infinite, NaN, zero
+// divisors, divisors past a reciprocal table): one quotient bit a step.  It is
+// slow on purpose: it keeps few values alive, where the FP64 unit's division
+// (or gxe_div) inlined here costs the whole kernel 8 to 17 registers.
+GXE_FN gxe_u64 gxe_div_rare(gxe_u64 a, gxe_u64 b) {
+  const gxe_u64 sign = (a ^ b) & GXE_SIGN;
+  a &= ~GXE_SIGN;
+  b &= ~GXE_SIGN;
+  if (a > GXE_INF || b > GXE_INF || (a == b && (a == 0 || a == GXE_INF))) return GXE_QNAN;
+  if (a == GXE_INF || b == 0) return sign | GXE_INF;
+  if (a == 0 || b == GXE_INF) return sign;
+  int e = (int)(a >> 52) - (int)(b >> 52);
+  gxe_u64 m = a & GXE_FRAC, d = b & GXE_FRAC;
+  if (a >> 52) m |= GXE_HIDDEN;
+  else e++;
+  if (b >> 52) d |= GXE_HIDDEN;
+  else e--;
+  while (!(m >> 52)) { m <<= 1; e--; }
+  while (!(d >> 52)) { d <<= 1; e++; }
+  if (m < d) { m <<= 1; e--; }
+  gxe_u64 q = 0;  // 55 bits, the first one set
+#if GXE_ON_DEVICE
+#pragma unroll 1
+#endif
+  for (int i = 0; i < 55; i++) {
+    q <<= 1;
+    if (m >= d) { m -= d; q |= 1ull; }
+    m <<= 1;
+  }
+  return gxe_round_pack(sign, e, q, m != 0);
+}
+
+// x / b for a literal b (normal, finite), r = gxe_recip_floor(b's significand)
+GXE_FN gxe_u64 gxe_div_lit(gxe_u64 a, gxe_u64 b, gxe_u64 r) {
+  const int ea = (int)((a >> 52) & 0x7FF), eb = (int)((b >> 52) & 0x7FF);
+  // x normal and the quotient's exponent (or one less) normal too
+  const int lo = eb > 1022 ? eb - 1021 : 1, hi = eb < 1023 ? eb + 1023 : 2046;
+  if ((unsigned)(ea - lo) > (unsigned)(hi - lo)) return (a << 1) == 0 ? (a ^ b) & GXE_SIGN : gxe_div_rare(a, b);
+  const gxe_u64 A = ((a & GXE_FRAC) | GXE_HIDDEN) << 11;
+  return gxe_quot((a ^ b) & GXE_SIGN, ea - eb + 1023, A, (b & GXE_FRAC) | GXE_HIDDEN, r);
+}
+
+// (double)x / b for a literal b and an integer x: as gxe_div_lit, without the
+// conversion (an x of more than 53 significant bits converts first)
+GXE_FN gxe_u64 gxe_divi_lit(gxe_i64 x, gxe_u64 b, gxe_u64 r) {
+  const int eb = (int)((b >> 52) & 0x7FF);
+  const gxe_u64 u = x < 0 ? 0ull - (gxe_u64)x : (gxe_u64)x;
+  const gxe_u64 sign = ((gxe_u64)x ^ b) & GXE_SIGN;
+  const int lz = gxe_clz(u);
+  const gxe_u64 A = u << (lz & 63);
+  const int e = 1023 + 63 - lz - eb + 1023;
+  if (u == 0) return sign;
+  if ((A & 0x7FFull) != 0 || (unsigned)(e - 2) > 2044u) return gxe_div_rare(gxe_i2d(x), b);
+  return gxe_quot(sign, e, A, (b & GXE_FRAC) | GXE_HIDDEN, r);
+}
+
+// x / k for an integer k: rcp[i] = gxe_recip_floor(significand of i + 1),
+// used for 1 <= |k| <= n.  Zeros of either side are answered here: a filter's
+// idle lanes divide 0 by 0, and must not draw their warp into the rare path.
+GXE_FN gxe_u64 gxe_div_k(gxe_u64 a, gxe_i64 k, const gxe_u64* rcp, int n) {
+  const gxe_u64 uk = k < 0 ? 0ull - (gxe_u64)k : (gxe_u64)k;
+  const int ea = (int)((a >> 52) & 0x7FF);
+  // n < 2^20: the quotient's exponent stays normal for ea in [32, 2046]
+  if (uk - 1ull >= (gxe_u64)n || (unsigned)(ea - 32) > 2014u) {
+    const bool zero = (a << 1) == 0;
+    if (k == 0 && !gxe_isnan_(a)) return zero ? GXE_QNAN : (a & GXE_SIGN) | GXE_INF;
+    if (zero) return a ^ ((gxe_u64)k & GXE_SIGN);
+    return gxe_div_rare(a, gxe_i2d(k));
+  }
+  const int lz = gxe_clz(uk);
+#if GXE_ON_DEVICE
+  const gxe_u64 r = __ldg(rcp + (uk - 1ull));
+#else
+  const gxe_u64 r = rcp[uk - 1ull];
+#endif
+  const gxe_u64 A = ((a & GXE_FRAC) | GXE_HIDDEN) << 11;
+  return gxe_quot((a ^ (gxe_u64)k) & GXE_SIGN, ea - (63 - lz), A, uk << (lz - 11), r);
+}
+
+// (double)x / (double)k for integers: as gxe_div_k, without the conversions
+GXE_FN gxe_u64 gxe_divi_k(gxe_i64 x, gxe_i64 k, const gxe_u64* rcp, int n) {
+  const gxe_u64 uk = k < 0 ? 0ull - (gxe_u64)k : (gxe_u64)k;
+  const gxe_u64 u = x < 0 ? 0ull - (gxe_u64)x : (gxe_u64)x;
+  const int lx = gxe_clz(u);
+  const gxe_u64 A = u << (lx & 63);
+  if (uk - 1ull >= (gxe_u64)n || u == 0 || (A & 0x7FFull) != 0) {
+    if (k == 0) return u == 0 ? GXE_QNAN : ((gxe_u64)x & GXE_SIGN) | GXE_INF;
+    if (u == 0) return (gxe_u64)k & GXE_SIGN;
+    return gxe_div_rare(gxe_i2d(x), gxe_i2d(k));
+  }
+  const int lz = gxe_clz(uk);
+#if GXE_ON_DEVICE
+  const gxe_u64 r = __ldg(rcp + (uk - 1ull));
+#else
+  const gxe_u64 r = rcp[uk - 1ull];
+#endif
+  return gxe_quot(((gxe_u64)x ^ (gxe_u64)k) & GXE_SIGN, 1023 + lz - lx, A, uk << (lz - 11), r);
+}
+
+// (double)v of an integer known to fit 32 bits: one shift instead of the
+// 64-bit normalisation and rounding of gxe_i2d
+GXE_FN gxe_u64 gxe_i2d32(int v) {
+  const unsigned u = v < 0 ? 0u - (unsigned)v : (unsigned)v;
+#if GXE_ON_DEVICE
+  const int lz = __clz((int)u);
+#else
+  const int lz = u ? __builtin_clz(u) : 32;
+#endif
+  const unsigned m = u << (lz & 31);
+  const unsigned hi = ((unsigned)(1023 + 30 - lz) << 20) + (m >> 11) + ((unsigned)v & 0x80000000u);
+  return u == 0 ? 0ull : ((gxe_u64)hi << 32) | (gxe_u64)(m << 21);
+}
+
+// round half away from zero (exact), as bits
+GXE_FN gxe_u64 gxe_round(gxe_u64 a) {
+  const int e = (int)((a >> 52) & 0x7FF) - 1023;
+  if (e >= 52) return (a & ~GXE_SIGN) > GXE_INF ? (a | (1ull << 51)) : a;  // integral, inf, nan
+  if (e < 0) return (a & GXE_SIGN) | (e == -1 ? 0x3FF0000000000000ull : 0ull);
+  a += (GXE_HIDDEN >> 1) >> e;  // half a unit, in magnitude
+  return a & ~(GXE_FRAC >> e);
+}
+
+// comparisons with a literal c (not NaN): ranges of the other operand's bits,
+// two 64-bit integer compares each
+GXE_FN bool gxe_ltc(gxe_u64 x, gxe_u64 c) {  // x < c
+  if ((c << 1) == 0) return x > GXE_SIGN && x <= (GXE_SIGN | GXE_INF);
+  if (c & GXE_SIGN) return x > c && x <= (GXE_SIGN | GXE_INF);
+  return (gxe_i64)x < (gxe_i64)c && x <= (GXE_SIGN | GXE_INF);
+}
+GXE_FN bool gxe_gtc(gxe_u64 x, gxe_u64 c) {  // x > c
+  if ((c << 1) == 0) return x - 1ull < GXE_INF;
+  if (c & GXE_SIGN) return x < c && (x <= GXE_INF || x >= GXE_SIGN);
+  return (gxe_i64)x > (gxe_i64)c && (gxe_i64)x <= (gxe_i64)GXE_INF;
+}
+GXE_FN bool gxe_eqc(gxe_u64 x, gxe_u64 c) { return (c << 1) == 0 ? (x << 1) == 0 : x == c; }
+GXE_FN bool gxe_lec(gxe_u64 x, gxe_u64 c) {  // x <= c
+  if ((c << 1) == 0) return x == 0 || (x >= GXE_SIGN && x <= (GXE_SIGN | GXE_INF));
+  if (c & GXE_SIGN) return x >= c && x <= (GXE_SIGN | GXE_INF);
+  return (gxe_i64)x <= (gxe_i64)c && x <= (GXE_SIGN | GXE_INF);
+}
+GXE_FN bool gxe_gec(gxe_u64 x, gxe_u64 c) {  // x >= c
+  if ((c << 1) == 0) return x <= GXE_INF || x == GXE_SIGN;
+  if (c & GXE_SIGN) return x <= c && (x <= GXE_INF || x >= GXE_SIGN);
+  return (gxe_i64)x >= (gxe_i64)c && (gxe_i64)x <= (gxe_i64)GXE_INF;
+}
+
 GXE_FN bool gxe_isnan(gxe_u64 a) { return (a & ~GXE_SIGN) > GXE_INF; }
 
 // total order key for non-NaN values with -0 == +0

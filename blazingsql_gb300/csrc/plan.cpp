@@ -4,7 +4,9 @@
 #include "fp64emu.cuh"
 
 #include <algorithm>
+#include <cmath>
 #include <cstdio>
+#include <cstdlib>
 #include <cstring>
 #include <functional>
 #include <map>
@@ -217,6 +219,12 @@ std::string raw_type(int t) {
   }
 }
 
+double bits_double(uint64_t u) {
+  double d;
+  std::memcpy(&d, &u, 8);
+  return d;
+}
+
 uint64_t magic_double_bits() {
   const double m = 1.7976931348623123e+308;  // interpreter_ops.cuh:47
   uint64_t u;
@@ -253,15 +261,63 @@ class Gen {
     return "v" + std::to_string(id) + "[k]";
   }
   bool kind_f(int id) const { return is_float(p_.nodes[id].ktype); }
+  // Bound on an integer-kind node's values: |v| < 2^bits (64: none known).
+  // Plans do not narrow at CASTs, so a CAST keeps its operand's bound; data
+  // under NULL is bounded like any other (columns are sign- or zero-extended
+  // from their storage type, and an unselected row reads 0).
+  int int_bits(int id) const {
+    const Node& n = p_.nodes[id];
+    if (kind_f(id)) return 64;
+    if (n.kind == Node::LIT) {
+      const int64_t v = n.lit_valid ? (int64_t)n.lit_bits : 0;
+      const uint64_t u = v < 0 ? 0ull - (uint64_t)v : (uint64_t)v;
+      return u == 0 ? 1 : 64 - __builtin_clzll(u);
+    }
+    if (n.kind == Node::COL) {
+      switch (p_.schema[n.col]) {
+        case INT8: case UINT8: case BOOL8: return 8;
+        case INT16: case UINT16: return 16;
+        case INT32: case UINT32: case TIMESTAMP_DAYS: case DURATION_DAYS: return 32;
+        default: return 64;
+      }
+    }
+    switch (n.op) {
+      case OP_EQ: case OP_NE: case OP_LT: case OP_GT: case OP_LE: case OP_GE: case OP_AND: case OP_NOT:
+      case OP_IS_NULL: case OP_IS_NOT_NULL: case OP_IS_NOT_TRUE: case OP_IS_NOT_FALSE:
+      case OP_IS_NOT_DISTINCT_FROM:
+        return 1;
+      case OP_CAST_TINYINT: case OP_CAST_SMALLINT: case OP_CAST_INTEGER: case OP_CAST_BIGINT: case OP_ABS:
+        return int_bits(n.a);
+      case OP_MOD:
+        if (kind_f(n.a) || kind_f(n.b)) return 64;
+        return p_.nodes[n.b].kind == Node::LIT ? std::min(int_bits(n.a), int_bits(n.b)) : int_bits(n.a);
+      case OP_ADD: case OP_SUB:
+        if (kind_f(n.a) || kind_f(n.b)) return 64;
+        return std::min(64, std::max(int_bits(n.a), int_bits(n.b)) + 1);
+      case OP_MUL:
+        if (kind_f(n.a) || kind_f(n.b)) return 64;
+        return std::min(64, int_bits(n.a) + int_bits(n.b));
+      default: return 64;
+    }
+  }
+  // (double) of an integer-kind node on the integer pipes, as bits; 31 bits
+  // and a sign (INT32's lowest value included) take the 32-bit form
+  std::string int_to_double(int id) const {
+    const Node& n = p_.nodes[id];
+    if (n.kind == Node::LIT) return hex64(n.lit_valid ? literal_double_bits(id) : 0ull);
+    const bool i32 = n.kind == Node::COL && p_.schema[n.col] != UINT32 && int_bits(id) <= 32;
+    if (i32 || int_bits(id) <= 31) return "gxe_i2d32((int)(" + B(id) + "))";
+    return "gxe_i2d((i64)(" + B(id) + "))";
+  }
   // operand as a double value (native FP64 arithmetic follows)
   std::string asD(int id) const {
     if (kind_f(id)) return "gx_D(" + B(id) + ")";
-    return emu_op(kNativeConvert) ? "gx_D(gxe_i2d((i64)(" + B(id) + ")))" : "gx_I2D(" + B(id) + ")";
+    return emu_op(kNativeConvert) ? "gx_D(" + int_to_double(id) + ")" : "gx_I2D(" + B(id) + ")";
   }
   // operand as the bits of its double value (integer-pipe binary64 routines follow)
   std::string asDB(int id) const {
     if (kind_f(id)) return B(id);
-    return emu_op(kNativeConvert) ? "gxe_i2d((i64)(" + B(id) + "))" : "gx_B(gx_I2D(" + B(id) + "))";
+    return emu_op(kNativeConvert) ? int_to_double(id) : "gx_B(gx_I2D(" + B(id) + "))";
   }
   std::string asI(int id) const {
     if (!kind_f(id)) return "(i64)(" + B(id) + ")";
@@ -269,7 +325,7 @@ class Gen {
   }
   std::string nz(int id) const {
     if (!kind_f(id)) return "(" + B(id) + " != 0ull)";
-    return emu_op(kNativeCompare) ? "gxe_nz(" + B(id) + ")" : "(gx_D(" + B(id) + ") != 0.0)";
+    return emu() ? "gxe_nz(" + B(id) + ")" : "(gx_D(" + B(id) + ") != 0.0)";
   }
   bool emu() const { return cfg_.emulate_fp64; }
   // this class of binary64 operation runs on the integer pipes
@@ -281,34 +337,38 @@ class Gen {
     const Node& n = p_.nodes[id];
     return kind_f(id) ? n.lit_bits : gxe_i2d((gxe_i64)n.lit_bits);
   }
-  // A divisor whose value is an integer (an integer-kind node, or its CAST
-  // to DOUBLE / FLOAT, which keeps the exact value inside a plan): the node
-  // holding that integer, or -1.  Divisions by it may take the reciprocal
-  // table (gxe_div_small) when the plan puts literal divisions on the FMA unit.
-  int int_divisor(int y) const {
+  // A node whose value is an integer (an integer-kind node, or its CAST to
+  // DOUBLE / FLOAT, which keeps the exact value inside a plan): the node
+  // holding that integer, or -1.  A CAST whose data under NULL is observable
+  // reads as 0 there, which the integer would not, so it counts as a double.
+  int int_source(int y) const {
     const Node& n = p_.nodes[y];
     if (n.kind == Node::LIT) return -1;
     if (!kind_f(y)) return y;
-    if (n.kind == Node::OP && (n.op == OP_CAST_DOUBLE || n.op == OP_CAST_FLOAT) && !kind_f(n.a) &&
+    if (n.kind == Node::OP && (n.op == OP_CAST_DOUBLE || n.op == OP_CAST_FLOAT) && !kind_f(n.a) && !n.exact_null &&
         p_.nodes[n.a].kind != Node::LIT)
       return n.a;
     return -1;
   }
+  // a division by an integer value reads the divisor's reciprocal from a table
   bool small_div(int id) const {
     const Node& n = p_.nodes[id];
     return n.kind == Node::OP && n.op == OP_DIV && (kind_f(n.a) || kind_f(n.b)) && emu_op(kNativeDiv) &&
-           !emu_op(kNativeIntDiv) && !const_divisor(n.b) && int_divisor(n.b) >= 0;
+           !const_divisor(n.b) && int_source(n.b) >= 0;
   }
-  // the reciprocal table gxe_div_small reads, when some division of the plan uses it
+  // The reciprocal table of the plan's divisions by an integer value, when it
+  // has one: 64-bit reciprocals of the integers' significands rounded down
+  // (gxe_div_k), or RN(1 / k) as binary64 (gxe_div_small on the FMA unit).
   void emit_rcp_table(std::ostringstream& o) const {
     bool any = false;
     for (size_t i = 0; i < p_.nodes.size() && !any; i++) any = small_div((int)i);
     if (!any) return;
     o << "#define GX_RCP_N " << kRcpTable << "\n__device__ const unsigned long long gx_rcp_[GX_RCP_N] = {";
     for (int k = 1; k <= kRcpTable; k++) {
-      const double y = 1.0 / (double)k;
+      double y = emu_op(kNativeIntDiv) ? (double)k : 1.0 / (double)k;
       uint64_t b;
       std::memcpy(&b, &y, 8);
+      if (emu_op(kNativeIntDiv)) b = gxe_recip_floor((b & GXE_FRAC) | GXE_HIDDEN);
       o << (k > 1 ? "," : "") << (k % 8 == 1 ? "\n  " : "") << hex64(b);
     }
     o << "};\n";
@@ -412,7 +472,10 @@ class Gen {
                           : op == OP_HOUR ? 4 : op == OP_MINUTE ? 5 : 6;
           const long long per_day = lt == TIMESTAMP_DAYS ? 1LL : 86400000000000LL / ns_per_unit(lt);
           const std::string cnt = lt == TIMESTAMP_DAYS ? "gx_days32((i64)(" + X + "))" : "(i64)(" + X + ")";
-          r = "(u64)gx_extract(" + cnt + ", " + std::to_string(per_day) + "LL, " + std::to_string(which) + ")";
+          if (per_day == 1 && which <= 2)  // a DATE's parts in 32-bit arithmetic
+            r = "(u64)gx_civil32((int)(" + X + "), " + std::to_string(which) + ")";
+          else
+            r = "(u64)gx_extract(" + cnt + ", " + std::to_string(per_day) + "LL, " + std::to_string(which) + ")";
           break;
         }
         case OP_CAST_TINYINT: case OP_CAST_SMALLINT: case OP_CAST_INTEGER: case OP_CAST_BIGINT:
@@ -490,6 +553,13 @@ class Gen {
         };
         return std::string("(u64)(") + to_ns(x, lt) + " " + opstr + " " + to_ns(y, rt) + ")";
       }
+      if (anyf && emu() && p_.nodes[y].kind == Node::LIT && p_.nodes[y].lit_valid && kind_f(x) &&
+          !gxe_isnan_(literal_double_bits(y))) {  // ranges of x's bits: no FP64-pipe compare
+        const std::string C = hex64(literal_double_bits(y)), o2 = opstr;
+        if (o2 == "!=") return "(u64)(!gxe_eqc(" + X + ", " + C + "))";
+        return "(u64)" + std::string(o2 == "<" ? "gxe_ltc(" : o2 == ">" ? "gxe_gtc(" : o2 == "<=" ? "gxe_lec("
+                                     : o2 == ">=" ? "gxe_gec(" : "gxe_eqc(") + X + ", " + C + ")";
+      }
       if (anyf && emu_op(kNativeCompare)) {
         const std::string X2 = asDB(x), Y2 = asDB(y), o2 = opstr;
         if (o2 == "<") return "(u64)gxe_lt(" + X2 + ", " + Y2 + ")";
@@ -531,28 +601,51 @@ class Gen {
           r = "gxe_div_c(" + asDB(x) + ", " + hex64(db) + ", " + hex64(gxe_recip_fixed((db & GXE_FRAC) | GXE_HIDDEN)) +
               ", " + hex64(yb) + ", " + std::to_string(lo) + ", " + std::to_string(hi) + ")";
         } else if (small_div(id)) {  // an integer divisor: RN(1/|k|) from the table for small |k|
-          r = "gxe_div_small(" + asDB(x) + ", (i64)(" + B(int_divisor(y)) + "), gx_rcp_, GX_RCP_N)";
+          const std::string k = "(i64)(" + B(int_source(y)) + "), gx_rcp_, GX_RCP_N)";
+          if (!emu_op(kNativeIntDiv)) r = "gxe_div_small(" + asDB(x) + ", " + k;
+          else if (int_source(x) >= 0) r = "gxe_divi_k((i64)(" + B(int_source(x)) + "), " + k;
+          else r = "gxe_div_k(" + asDB(x) + ", " + k;
         } else if (anyf && emu_op(kNativeDiv) && const_divisor(y)) {
-          // constant divisor: its fixed-point reciprocal is computed here
+          // constant divisor: its reciprocal is computed here
           const uint64_t db = literal_double_bits(y);
-          r = "gxe_div_r(" + asDB(x) + ", " + hex64(db) + ", " +
-              hex64(gxe_recip_fixed((db & GXE_FRAC) | GXE_HIDDEN)) + ")";
+          const std::string c = hex64(db) + ", " + hex64(gxe_recip_floor((db & GXE_FRAC) | GXE_HIDDEN)) + ")";
+          r = int_source(x) >= 0 ? "gxe_divi_lit((i64)(" + B(int_source(x)) + "), " + c : "gxe_div_lit(" + asDB(x) + ", " + c;
         } else {
           r = !anyf ? "gx_div_ii(" + X + ", " + Y + ")"
               : emu_op(kNativeDiv) ? "gxe_div(" + asDB(x) + ", " + asDB(y) + ")" : "gx_B(" + asD(x) + " / " + asD(y) + ")";
         }
-        vv = "(" + vv + " && " + (rf ? nz(y) : "(i64)(" + Y + ") != 0LL") + ")";
+        if (const_divisor(y)) break;  // never zero
+        if (rf && emu() && int_source(y) >= 0) vv = "(" + vv + " && (i64)(" + B(int_source(y)) + ") != 0LL)";
+        else vv = "(" + vv + " && " + (rf ? nz(y) : "(i64)(" + Y + ") != 0LL") + ")";
         break;
       case OP_MOD:
         if (anyf) {
           r = "gx_B(fmod(" + asD(x) + ", " + asD(y) + "))";
+        } else if (int_bits(x) <= 31 && int_bits(y) <= 31) {  // 32-bit remainder
+          r = "gx_mod_32((int)(" + X + "), (int)(" + Y + "))";
+          vv = "(" + vv + " && (i64)(" + Y + ") != 0LL)";
         } else {
           r = "gx_mod_ii(" + X + ", " + Y + ")";
           vv = "(" + vv + " && (i64)(" + Y + ") != 0LL)";
         }
         break;
       case OP_POW: r = "gx_B(pow(" + asD(x) + ", " + asD(y) + "))"; break;
-      case OP_ROUND: r = "gx_B(gx_round_to(" + asD(x) + ", " + asD(y) + "))"; break;
+      case OP_ROUND: {
+        // a literal integral digit count of at most 22: the scale is the
+        // literal 10^d, the rounding and the division stay on the integer pipes
+        const double d = p_.nodes[y].kind == Node::LIT && p_.nodes[y].lit_valid ? bits_double(literal_double_bits(y)) : 99.0;
+        if (emu_op(kNativeDiv) && emu_op(kNativeRound) && d >= -22.0 && d <= 22.0 && d == std::floor(d)) {
+          const std::string f = "1e" + std::to_string((int)d);
+          const double fv = std::strtod(f.c_str(), nullptr);
+          uint64_t fb;
+          std::memcpy(&fb, &fv, 8);
+          r = "gxe_div_lit(gxe_round(gx_B(" + asD(x) + " * gx_D(" + hex64(fb) + "))), " + hex64(fb) + ", " +
+              hex64(gxe_recip_floor((fb & GXE_FRAC) | GXE_HIDDEN)) + ")";
+        } else {
+          r = "gx_B(gx_round_to(" + asD(x) + ", " + asD(y) + "))";
+        }
+        break;
+      }
       case OP_EQ: r = cmp("=="); break;
       case OP_NE: r = cmp("!="); break;
       case OP_LT: r = cmp("<"); break;
@@ -2161,36 +2254,21 @@ std::vector<int> conjunct_columns(const Plan& p, int c) {
 
 // Which binary64 operation classes go to the FP64 pipe when the plan leaves it
 // to the library.  Both forms are exact; the choice balances the two pipes.
-// Add, subtract and multiply cost about as much natively (one FP64-pipe
-// instruction, at 1/64 of the FP32 rate) as emulated (about 25 integer
-// instructions), so moving them to the otherwise idle FP64 pipe frees the
-// integer pipes.  Integer-to-double conversions go there too.  Compares go
-// there only when the plan has no transcendental (LN / EXP / trigonometric /
-// POWER / ROUND, which already load the FP64 pipe): with one they cost more
-// time there than they free.  So does division by a literal (a multiply and
-// two FMAs instead of about 100 integer instructions).  Other division stays
-// emulated: natively it is a reciprocal and Newton steps, several FP64-pipe
-// instructions.  Measured on
-// GB300 against all-emulated: 25 % on the deep plan (with LN / EXP; the
-// conversions are 6.5 % of it), 10 % on the plain filter + divide.
-int auto_native_f64_ops(const Plan& p) {
-  bool transcendental = false;
-  for (const auto& n : p.nodes)
-    if (n.kind == Node::OP) switch (n.op) {
-        case OP_SIN: case OP_COS: case OP_ASIN: case OP_ACOS: case OP_TAN: case OP_COTAN: case OP_ATAN:
-        case OP_LN: case OP_LOG10: case OP_EXP: case OP_POW: case OP_ROUND:
-          transcendental = true;
-          break;
-        default: break;
-      }
-  return transcendental ? (kNativeAddSub | kNativeMul | kNativeConvert)
-                        : (kNativeAddSub | kNativeMul | kNativeConvert | kNativeCompare | kNativeConstDiv |
-                           kNativeIntDiv);
-}
+// The FP64 pipe takes a warp instruction every 16 clocks per SM, the ALU and
+// IMAD pipes two a clock each.  Add, subtract and multiply are one FP64
+// instruction or about 25 integer ones (12 clocks), close enough that the
+// otherwise idle FP64 pipe takes them.  Conversions (10 to 20 integer
+// instructions), compares with a literal (4) and divisions by a literal or an
+// integer (about 30, against a multiply, two FMAs and the conversions of the
+// operands) are far cheaper on the integer pipes: with them there, against all
+// of them on the FP64 pipe, the order-line plan at 2^27 rows takes 2.43 ms
+// instead of 2.83, its aggregation at 2^26 2.14 instead of 2.45, the deep plan
+// at 2^26 1.70 instead of 1.82.
+int auto_native_f64_ops() { return kNativeAddSub | kNativeMul; }
 
 std::string generate_kernel(const Plan& p, KernelKind kind, const KernelConfig& cfg_in, const std::string& name) {
   KernelConfig cfg = cfg_in;
-  if (cfg.native_f64_ops < 0) cfg.native_f64_ops = auto_native_f64_ops(p);
+  if (cfg.native_f64_ops < 0) cfg.native_f64_ops = auto_native_f64_ops();
   Gen g(p, cfg);
   if (p.has_filter() && cfg.dense) {
     // columns whose data the predicate reads (not only their validity, as
@@ -2373,11 +2451,7 @@ uint64_t agg_counts_are_rows(const Plan& p, const AggLayout& L) {
 std::string generate_agg_kernel(const Plan& p, const AggLayout& L, const KernelConfig& cfg_in,
                                 const std::string& name) {
   KernelConfig cfg = cfg_in;
-  // the aggregation's floating sums and combining trees already load the FP64
-  // pipe: divisions stay on the integer pipes (Q1 shape: 3.72 ms, against
-  // 3.93 ms with the literal division and 3.91 ms with the integer-value
-  // division on the FMA unit)
-  if (cfg.native_f64_ops < 0) cfg.native_f64_ops = auto_native_f64_ops(p) & ~(kNativeConstDiv | kNativeIntDiv);
+  if (cfg.native_f64_ops < 0) cfg.native_f64_ops = auto_native_f64_ops();
   cfg.short_circuit = false;
   cfg.runtime_order = false;
   cfg.conjunct_order.clear();
