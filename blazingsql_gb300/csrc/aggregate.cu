@@ -298,11 +298,7 @@ void AggPlan::execute(const std::vector<ColumnView>& cols, gx_column* out, int64
       }
       if (n > 0) {
         KernelArgs a{};
-        for (size_t i = 0; i < cols.size(); i++) {
-          a.in_data[i] = cols[i].data;
-          a.in_mask[i] = cols[i].mask;
-          a.in_off[i] = cols[i].offset;
-        }
+        for (size_t i = 0; i < cols.size(); i++) bind_column(a, i, cols[i]);
         a.n = n;
         a.tile_counter = flags + 3;
         a.err = t.err;

@@ -191,11 +191,7 @@ int64_t BatchRunner::stage(const std::vector<std::vector<ColumnView>>& batches, 
     std::memset(&a, 0, sizeof a);
     const auto& cols = batches[b];
     const int64_t n = cols.empty() ? 0 : cols[0].size;
-    for (size_t i = 0; i < cols.size(); i++) {
-      a.in_data[i] = cols[i].data;
-      a.in_mask[i] = cols[i].mask;
-      a.in_off[i] = cols[i].offset;
-    }
+    for (size_t i = 0; i < cols.size(); i++) bind_column(a, i, cols[i]);
     for (int j = 0; j < nout; j++) {
       a.out_data[j] = out[(size_t)b * nout + j].data;
       a.out_mask[j] = out[(size_t)b * nout + j].null_mask;
@@ -557,11 +553,7 @@ int BatchStream::push(const std::vector<ColumnView>& cols) {
   const int nout = num_outputs();
   KernelArgs& a = *(KernelArgs*)((char*)hargs_ + (size_t)b * kStreamArgsStride);
   std::memset(&a, 0, sizeof a);
-  for (size_t i = 0; i < cols.size(); i++) {
-    a.in_data[i] = cols[i].data;
-    a.in_mask[i] = cols[i].mask;
-    a.in_off[i] = cols[i].offset;
-  }
+  for (size_t i = 0; i < cols.size(); i++) bind_column(a, i, cols[i]);
   for (int j = 0; j < nout; j++) {
     a.out_data[j] = arena_ + doff_[j] + (size_t)rows_used_ * type_size(plan_.outputs[j].type);
     a.out_mask[j] = (uint32_t*)(arena_ + moff_[j]) + rows_used_ / 32;

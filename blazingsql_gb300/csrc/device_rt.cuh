@@ -128,6 +128,47 @@ __device__ __forceinline__ bool gx_valid(const u32* __restrict__ m, i64 bit) {
   return m == nullptr ? true : ((__ldg(m + (bit >> 5)) >> (bit & 31)) & 1u);
 }
 
+// Validity word w of a batch's n rows (bit i: row 32 w + i), re-aligned from a
+// mask whose first row is bit `sh` (0..31) of word 0; no mask: all valid.  A
+// warp's lanes hold its tile's words this way (one coalesced load per column
+// and tile), and a row's bit comes by shuffle (gx_wbit) instead of an address
+// and a load per row.
+__device__ __forceinline__ u32 gx_mask_word(const u32* __restrict__ m, i64 sh, i64 w, i64 n) {
+  if (w * 32 >= n) return 0u;
+  if (m == nullptr) return GX_FULL;
+  const u32 lo = __ldg(m + w);
+  if (sh == 0) return lo;
+  const u32 hi = w * 32 + (32 - sh) < n ? __ldg(m + w + 1) : 0u;
+  return __funnelshift_r(lo, hi, (u32)sh);
+}
+// bit `i` of the word that lane `l` holds (every lane of the warp calls)
+__device__ __forceinline__ bool gx_wbit(u32 word, u32 l, u32 i) { return (__shfl_sync(GX_FULL, word, (int)l) >> i) & 1u; }
+
+// A warp's kept rows append `total` validity bits at bit position pos of an
+// output mask: lane r holds round r's bits (rows 32 r .. 32 r + 31 of the
+// range).  Words inside the range are stored; its first and last words, which
+// the neighbouring ranges share, are OR-ed (the mask was zeroed before the
+// launch).  Words at and past cap_words are not written.
+__device__ __forceinline__ void gx_put_bits(u32* mask, i64 pos, u32 total, u32 bits, i64 cap_words) {
+  const u32 lane = threadIdx.x & 31;
+  const u32 sh = (u32)pos & 31u, end = sh + total;
+  const i64 w = (pos >> 5) + lane;
+  u32 prev = __shfl_up_sync(GX_FULL, bits, 1);
+  if (lane == 0) prev = 0u;
+  const u32 v = __funnelshift_l(prev, bits, sh);
+  if (lane * 32u < end && w < cap_words) {
+    if ((lane == 0 && sh != 0u) || (lane + 1u) * 32u > end) atomicOr(mask + w, v);
+    else mask[w] = v;
+  }
+  // 32 full rounds at an odd position reach a 33rd word
+  if (lane == 31 && end > 1024u && w + 1 < cap_words) atomicOr(mask + w + 1, bits >> (32u - sh));
+}
+// lane r's bits for `total` rows that are all valid
+__device__ __forceinline__ u32 gx_ones(u32 total) {
+  const int left = (int)total - (int)(threadIdx.x & 31) * 32;
+  return left >= 32 ? GX_FULL : left <= 0 ? 0u : (1u << left) - 1u;
+}
+
 // ---- streaming loads / stores ------------------------------------------------
 __device__ __forceinline__ i64 gx_ld_i8(const void* p, i64 i) { return (i64)__ldcs((const signed char*)p + i); }
 __device__ __forceinline__ i64 gx_ld_u8(const void* p, i64 i) { return (i64)__ldcs((const unsigned char*)p + i); }

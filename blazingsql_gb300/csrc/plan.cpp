@@ -244,7 +244,27 @@ int64_t ns_per_unit(int t) {
 
 class Gen {
  public:
-  Gen(const Plan& p, const KernelConfig& c) : p_(p), cfg_(c) {}
+  Gen(const Plan& p, const KernelConfig& c) : p_(p), cfg_(c) {
+    for (int r : p.conjuncts) prove_valid(r);
+  }
+
+  // Columns that are valid in every row a conjunct keeps: a kept row's
+  // conjunct is valid and true, and an operator that is NULL whenever an
+  // operand is makes its operands valid too.
+  void prove_valid(int id) {
+    const Node& n = p_.nodes[id];
+    if (n.kind == Node::COL) { proven_.insert(n.col); return; }
+    if (n.kind != Node::OP) return;
+    switch (n.op) {
+      case OP_IS_NOT_NULL: prove_valid(n.a); return;
+      case OP_OR: case OP_IS_NULL: case OP_IS_TRUE: case OP_IS_NOT_TRUE: case OP_IS_NOT_FALSE:
+      case OP_IS_NOT_DISTINCT_FROM: case OP_MAGIC_IF_NOT: case OP_FIRST_NON_MAGIC: case OP_RAND: case OP_ROW_INDEX:
+        return;
+      default: break;
+    }
+    if (n.a >= 0) prove_valid(n.a);
+    if (n.b >= 0) prove_valid(n.b);
+  }
 
   // operand views for node id in word-slot k
   std::string B(int id) const { return value_bits(id); }
@@ -363,15 +383,21 @@ class Gen {
     bool any = false;
     for (size_t i = 0; i < p_.nodes.size() && !any; i++) any = small_div((int)i);
     if (!any) return;
+    static const std::string tables[2] = {rcp_table(false), rcp_table(true)};
+    o << tables[emu_op(kNativeIntDiv) ? 1 : 0];
+  }
+  static std::string rcp_table(bool fixed) {
+    std::ostringstream o;
     o << "#define GX_RCP_N " << kRcpTable << "\n__device__ const unsigned long long gx_rcp_[GX_RCP_N] = {";
     for (int k = 1; k <= kRcpTable; k++) {
-      double y = emu_op(kNativeIntDiv) ? (double)k : 1.0 / (double)k;
+      const double y = fixed ? (double)k : 1.0 / (double)k;
       uint64_t b;
       std::memcpy(&b, &y, 8);
-      if (emu_op(kNativeIntDiv)) b = gxe_recip_floor((b & GXE_FRAC) | GXE_HIDDEN);
+      if (fixed) b = gxe_recip_floor((b & GXE_FRAC) | GXE_HIDDEN);
       o << (k > 1 ? "," : "") << (k % 8 == 1 ? "\n  " : "") << hex64(b);
     }
     o << "};\n";
+    return o.str();
   }
   static constexpr int kRcpTable = 1024;
   // a literal divisor that is a normal finite nonzero double
@@ -380,6 +406,44 @@ class Gen {
     if (n.kind != Node::LIT || !n.lit_valid) return false;
     const int e = (int)((literal_double_bits(id) >> 52) & 0x7FF);
     return e >= 1 && e <= 2046;
+  }
+
+  // the load of a column's element at `row` (data pointers start at the batch's first row)
+  std::string load_call(int c) const {
+    std::string fn = emu() ? load_fn_emu(p_.schema[c]) : load_fn(p_.schema[c]);
+    if (reread_cols_.count(c)) fn = "gx_ldg_" + fn.substr(6);  // gx_ld_X -> gx_ldg_X
+    return fn + "(a.in_data[" + std::to_string(c) + "], row)";
+  }
+  // where a row's validity bit is read from
+  enum class Masks {
+    GLOBAL,  // the mask, by row
+    WORDS,   // lane l holds word l of the warp's words (mw_<c>); slot k, bit `lane`
+    KEPT,    // the same words; the row's offset within the warp's rows is kp_, and
+             // the condition has made the proven_ columns valid
+  };
+  mutable Masks masks_ = Masks::GLOBAL;
+  bool masked(int c) const { return p_.nullable[c] && !(masks_ == Masks::KEPT && proven_.count(c)); }
+  // validity of column c for the lane's row
+  std::string col_valid(int c) const {
+    const std::string cs = std::to_string(c);
+    if (!masked(c)) return "inr";
+    switch (masks_) {
+      case Masks::WORDS: return "(gx_wbit(mw_" + cs + ", k, lane) && inr)";
+      case Masks::KEPT: return "(gx_wbit(mw_" + cs + ", kp_ >> 5, kp_ & 31u) && inr)";
+      default: return "(inr && gx_valid(a.in_mask[" + cs + "], a.in_off[" + cs + "] + row))";
+    }
+  }
+  // the validity words that the rows of `ids` and of the columns `more` need,
+  // one word per lane (words w0 .. w0 + GX_V - 1)
+  void emit_mask_words(std::ostringstream& o, const std::vector<int>& ids, const std::vector<int>& more,
+                       const std::string& ind) const {
+    std::set<int> cols(more.begin(), more.end());
+    for (int id : ids)
+      if (p_.nodes[id].kind == Node::COL) cols.insert(p_.nodes[id].col);
+    for (int c : cols)
+      if (masked(c))
+        o << ind << "const u32 mw_" << c << " = lane < GX_V ? gx_mask_word(a.in_mask[" << c << "], a.in_off[" << c
+          << "], w0 + lane, a.n) : 0u;\n";
   }
 
   // statements computing node id for slot k; row / out-row expressions given
@@ -408,14 +472,11 @@ class Gen {
         const std::string gfn = emu() ? load_fn_emu(p_.schema[c]) : load_fn(p_.schema[c]);
         const std::string sfn = "gx_lds_" + gfn.substr(6);  // gx_ld_X -> gx_lds_X
         o << ind << b << " = inr ? (full_word_ ? (u64)" << sfn << "(" << st->second.first << ", " << st->second.second
-          << ") : (u64)" << gfn << "(a.in_data[" << c << "], a.in_off[" << c << "] + row)) : 0ull;\n";
+          << ") : (u64)" << gfn << "(a.in_data[" << c << "], row)) : 0ull;\n";
       } else {
-        std::string fn = emu() ? load_fn_emu(p_.schema[c]) : load_fn(p_.schema[c]);
-        if (reread_cols_.count(c)) fn = "gx_ldg_" + fn.substr(6);  // gx_ld_X -> gx_ldg_X
-        o << ind << b << " = inr ? (u64)" << fn << "(a.in_data[" << c << "], a.in_off[" << c << "] + row) : 0ull;\n";
+        o << ind << b << " = inr ? (u64)" << load_call(c) << " : 0ull;\n";
       }
-      if (p_.nullable[c]) o << ind << v << " = inr && gx_valid(a.in_mask[" << c << "], a.in_off[" << c << "] + row);\n";
-      else o << ind << v << " = inr;\n";
+      o << ind << v << " = " << col_valid(c) << ";\n";
       return;
     }
     std::string r, vv;
@@ -704,6 +765,11 @@ class Gen {
                    : "const i64 row = (w0 + k) * 32 + lane; const bool inr = " + inr + "; (void)inr;\n";
     bool any_col = false;
     for (int id : ids) any_col |= p_.nodes[id].kind == Node::COL;
+    const Masks was = masks_;
+    if (!tile_mode_) {
+      masks_ = Masks::WORDS;
+      emit_mask_words(o, ids, {}, ind);
+    }
     if (any_col) {
       o << ind << "#pragma unroll\n" << ind << "for (int k = 0; k < GX_V; k++) {\n" << ind << "  " << rowdef;
       for (int id : ids)
@@ -715,6 +781,7 @@ class Gen {
       if (p_.nodes[id].kind != Node::COL) emit_node(o, id, ind + "  ");
     if (!tail.empty()) o << ind << "  " << tail << "\n";
     o << ind << "}\n";
+    masks_ = was;
   }
 
   // predicate phase: fills keep bits bal[k]; with short-circuit, conjuncts are
@@ -727,7 +794,10 @@ class Gen {
       order = p_.conjuncts;
     }
     o << ind << "bool alive[GX_V];\n";
-    o << ind << "#pragma unroll\n" << ind << "for (int k = 0; k < GX_V; k++) alive[k] = (w0 + k) * 32 + lane < a.n;\n";
+    if (!tile_mode_)  // rows of the warp's words that exist, 0 .. 32 GX_V
+      o << ind << "const int nrow_ = (int)max(min(a.n - w0 * 32, (i64)(GX_V * 32)), (i64)0);\n";
+    o << ind << "#pragma unroll\n" << ind << "for (int k = 0; k < GX_V; k++) alive[k] = "
+      << (tile_mode_ ? "(w0 + k) * 32 + lane < a.n" : "k * 32 + lane < nrow_") << ";\n";
     if (cfg_.runtime_order) {
       if (cfg_.stream_slots > 0 && streamable())
         emit_predicate_stream(o, ind);
@@ -740,7 +810,7 @@ class Gen {
       // fixed order: evaluate every conjunct for every row
       std::string keep = "inr";
       for (int c : order) keep += " && " + conj_keep(c);
-      emit_words(o, cone(order), ind, "row < a.n", "alive[k] = " + keep + ";");
+      emit_words(o, cone(order), ind, tile_mode_ ? "row < a.n" : "k * 32 + lane < nrow_", "alive[k] = " + keep + ";");
       return;
     }
     o << ind << "bool any_alive = true;\n";
@@ -846,8 +916,8 @@ class Gen {
       const int col = col_of[c];
       if (col < 0) continue;
       const std::string gfn = emu() ? load_fn_emu(p_.schema[col]) : load_fn(p_.schema[col]);
-      o << ind << "      case " << c << ": val_[q] = inr ? (u64)" << gfn << "(a.in_data[" << col << "], a.in_off[" << col
-        << "] + row) : 0ull; vv_[q] = inr" << (p_.nullable[col] ? " && gx_valid(a.in_mask[" + std::to_string(col) +
+      o << ind << "      case " << c << ": val_[q] = inr ? (u64)" << gfn << "(a.in_data[" << col
+        << "], row) : 0ull; vv_[q] = inr" << (p_.nullable[col] ? " && gx_valid(a.in_mask[" + std::to_string(col) +
                                                                       "], a.in_off[" + std::to_string(col) + "] + row)"
                                                                 : std::string())
         << "; break;\n";
@@ -1021,14 +1091,15 @@ class Gen {
   // columns whose data both the predicate and the projections read: loaded
   // with the default cache policy so the projections' re-read hits L2
   mutable std::set<int> reread_cols_;
+  std::set<int> proven_;  // columns valid in every kept row (prove_valid)
 
-  // validity of node id is true for every row in range (no NULL can arise):
-  // non-nullable columns, valid literals, and operators that propagate only
+  // validity of node id is true for every row the filter keeps (no NULL can
+  // arise): non-nullable columns, columns the condition proves valid, valid literals, and operators that propagate only
   // their operands' validity or divide by a nonzero literal
   bool never_null(int id) const {
     const Node& n = p_.nodes[id];
     if (n.kind == Node::LIT) return n.lit_valid;
-    if (n.kind == Node::COL) return !p_.nullable[n.col];
+    if (n.kind == Node::COL) return !p_.nullable[n.col] || proven_.count(n.col);
     switch (n.op) {
       case OP_RAND: case OP_ROW_INDEX:
       case OP_IS_NOT_TRUE: case OP_IS_NOT_FALSE: case OP_IS_NULL: case OP_IS_NOT_NULL: case OP_IS_NOT_DISTINCT_FROM:
@@ -1082,10 +1153,8 @@ std::string emit_dense_store(std::ostringstream& o, const Gen& g, const Plan& p,
   if (os.kind != OutSpec::COPY) return "";
   const int c = os.col;
   const std::string rt = raw_type(p.schema[c]);
-  o << ind << "if (wr) ((" << rt << "*)a.out_data[" << j << "])[orow] = __ldcs((const " << rt << "*)a.in_data[" << c
-    << "] + a.in_off[" << c << "] + row);\n";
-  return p.nullable[c] ? "gx_valid(a.in_mask[" + std::to_string(c) + "], a.in_off[" + std::to_string(c) + "] + row)"
-                       : "true";
+  o << ind << "if (wr) __stcs((" << rt << "*)a.out_data[" << j << "] + orow, r" << j << "_);\n";
+  return g.col_valid(c);
 }
 
 // outputs that carry a validity bit stream (broadcasts are filled after the launch)
@@ -1096,15 +1165,10 @@ std::vector<size_t> masked_outputs(const Plan& p) {
   return v;
 }
 
-// Dense phase 2: the warp's kept rows, in row order, are dealt to lanes in
-// rounds of 32 (lane l of round r takes the warp's (32r + l)-th kept row), so
-// projections are computed only for surviving rows and every output store and
-// validity word of a round is contiguous.  Operands are re-read with the
-// gathered row index (predicate columns hit L1/L2).
 // statements mapping kept rank t_ of the warp (0 <= t_ < total_) to its row
 // through the warp's kept-row list in shared memory
 void emit_rank_to_row(std::ostringstream& o, const std::string& ind) {
-  o << ind << "const i64 row = w0 * 32 + (act ? (i64)s_kept_[warp][t_] : 0); const bool inr = act; (void)inr;\n";
+  o << ind << "const u32 kp_ = act ? (u32)s_kept_[warp][t_] : 0u; const i64 row = w0 * 32 + kp_; const bool inr = act; (void)inr;\n";
   o << ind << "const i64 orow = (i64)pos + (i64)t_; (void)orow;\n";
   o << ind << "const int k = 0;\n";
 }
@@ -1135,6 +1199,17 @@ void emit_row_nodes(std::ostringstream& o, const Gen& g, const Plan& p, const st
 // gathered row index (predicate columns hit L1/L2).  Expensive CASE branches
 // (Gen::lazy_branches) are first evaluated for the kept rows whose condition
 // selects them, packed into full warps, into shared memory.
+//
+// What bounds it is instructions and load latency (order-line plan, ncu: IPC
+// 1.7, 340 instructions per 32 rows, most of them addresses and validity).  So
+// a round keeps both small: columns share one row index (bind_column folds the
+// view's offset into the pointers); validity comes by shuffle from words that
+// the warp's lanes loaded once per tile, and not at all for columns that the
+// condition proves valid; output validity bits stay in lane r until the warp
+// has done its rounds, then go out one coalesced store per mask instead of one
+// lane's store per mask and round.  340 -> 285 instructions, call time at 2^27
+// rows 2.43 -> 2.08 ms; deep plan 2^26 1.70 -> 1.47; process_filter of six
+// columns 2^23 0.346 -> 0.274.
 void emit_filter_writes_dense(std::ostringstream& o, const Gen& g, const Plan& p, const std::string& ind) {
   const std::vector<int> roots = g.output_roots();
   const std::vector<Gen::Lazy> lz = g.lazy_branches(roots);
@@ -1145,6 +1220,14 @@ void emit_filter_writes_dense(std::ostringstream& o, const Gen& g, const Plan& p
     stop.insert(lz[i].root);
   }
   const std::vector<int> proj = g.cone_stop(roots, stop);
+  const Gen::Masks was = g.masks_;
+  g.masks_ = Gen::Masks::KEPT;
+  {
+    std::vector<int> copied;
+    for (const auto& os : p.outputs)
+      if (os.kind == OutSpec::COPY) copied.push_back(os.col);
+    g.emit_mask_words(o, g.cone(roots), copied, ind);
+  }
   // the warp's kept rows in order: offsets from its first row, by kept rank
   o << ind << "__shared__ unsigned short s_kept_[GX_WARPS][GX_V * 32];\n";
   o << ind << "u32 total_ = 0u;\n";
@@ -1201,59 +1284,45 @@ void emit_filter_writes_dense(std::ostringstream& o, const Gen& g, const Plan& p
     }
     o << ind << "__syncwarp();\n";
   }
-  // validity bit streams: one position shared by all outputs (every round
-  // appends the same number of bits to each), one accumulator per output
-  // whose validity varies and one shared by the outputs that are never NULL;
-  // the first word may be shared with the previous warp's range and the last
-  // with the next one (atomicOr), words in between are stored
+  // validity bits: lane r keeps round r's ballot of each output whose validity
+  // varies (outputs that are never NULL need none), and the warp writes every
+  // mask once, after its rounds (gx_put_bits)
   const std::vector<size_t> mo = masked_outputs(p);
   std::vector<int> slot(p.outputs.size(), -1);
-  int nslots = 0, nn_slot = -1;
+  int nslots = 0;
   for (size_t j : mo) {
     const OutSpec& os = p.outputs[j];
-    if (os.kind == OutSpec::COPY ? !p.nullable[os.col] : g.never_null(os.node)) {
-      if (nn_slot < 0) nn_slot = nslots++;
-      slot[j] = nn_slot;
-    } else {
-      slot[j] = nslots++;
-    }
+    if (os.kind == OutSpec::COPY ? g.masked(os.col) : !g.never_null(os.node)) slot[j] = nslots++;
   }
-  const int nacc = std::max(nslots, 1);
-  o << ind << "u64 acc_[" << nacc << "];\n";
-  o << ind << "#pragma unroll\n" << ind << "for (int j = 0; j < " << nacc << "; j++) acc_[j] = 0ull;\n";
-  o << ind << "int bf_ = (int)(pos & 31ull); i64 bword_ = (i64)(pos >> 5); bool bfirst_ = bf_ != 0;\n";
-  o << ind << "const i64 cap_words = (a.capacity + 31) >> 5;\n";
+  for (int sl = 0; sl < nslots; sl++) o << ind << "u32 vb" << sl << "_ = 0u;\n";
+  o << ind << "const u32 wmax_ = (u32)max((i64)0, min((i64)total_, a.capacity - (i64)pos));\n";
   o << ind << "for (u32 base_ = 0; base_ < total_; base_ += 32u) {\n";
   const std::string in2 = ind + "  ";
   o << in2 << "const u32 t_ = base_ + (u32)lane; const bool act = t_ < total_;\n";
   emit_rank_to_row(o, in2);
-  emit_row_nodes(o, g, p, proj, lz_root, in2);
-  o << in2 << "const bool wr = act && orow < a.capacity;\n";
-  o << in2 << "const int nb = (int)min(32u, total_ - base_);\n";
-  std::vector<std::string> vexpr(p.outputs.size());
-  for (size_t j = 0; j < p.outputs.size(); j++) vexpr[j] = emit_dense_store(o, g, p, j, in2);
-  for (int sl = 0; sl < nslots; sl++) {
-    std::string e = "act";
-    if (sl != nn_slot)
-      for (size_t j : mo)
-        if (slot[j] == sl) e = "act && " + vexpr[j];
-    o << in2 << "acc_[" << sl << "] |= (u64)__ballot_sync(GX_FULL, " << e << ") << bf_;\n";
+  // the copied columns' loads go out with the projections'
+  for (size_t j = 0; j < p.outputs.size(); j++) {
+    if (p.outputs[j].kind != OutSpec::COPY) continue;
+    const int c = p.outputs[j].col;
+    const std::string rt = raw_type(p.schema[c]);
+    o << in2 << "const " << rt << " r" << j << "_ = act ? " << (g.reread_cols_.count(c) ? "__ldg" : "__ldcs") << "((const "
+      << rt << "*)a.in_data[" << c << "] + row) : (" << rt << ")0;\n";
   }
-  o << in2 << "const int nf_ = bf_ + nb;\n";
-  o << in2 << "if (nf_ >= 32) {\n";
-  o << in2 << "  if (lane == 0 && bword_ < cap_words) {\n";
-  for (size_t j : mo)
-    o << in2 << "    if (bfirst_) atomicOr(a.out_mask[" << j << "] + bword_, (u32)acc_[" << slot[j] << "]); else a.out_mask["
-      << j << "][bword_] = (u32)acc_[" << slot[j] << "];\n";
-  o << in2 << "  }\n";
-  o << in2 << "  #pragma unroll\n" << in2 << "  for (int j = 0; j < " << nacc << "; j++) acc_[j] >>= 32;\n";
-  o << in2 << "  bfirst_ = false; bword_++; bf_ = nf_ - 32;\n";
-  o << in2 << "} else {\n" << in2 << "  bf_ = nf_;\n" << in2 << "}\n";
+  emit_row_nodes(o, g, p, proj, lz_root, in2);
+  o << in2 << "const bool wr = t_ < wmax_;\n";
+  for (size_t j = 0; j < p.outputs.size(); j++) {
+    const std::string v = emit_dense_store(o, g, p, j, in2);
+    if (slot[j] < 0) continue;
+    o << in2 << "{ const u32 b_ = __ballot_sync(GX_FULL, " << v << " && act); if ((u32)lane == base_ >> 5) vb" << slot[j]
+      << "_ = b_; }\n";
+  }
   o << ind << "}\n";
   o << ind << "__syncwarp();\n";  // the kept-row list and branch results are rewritten by the next tile
-  o << ind << "if (bf_ > 0 && lane == 0 && bword_ < cap_words) {\n";
-  for (size_t j : mo) o << ind << "  atomicOr(a.out_mask[" << j << "] + bword_, (u32)acc_[" << slot[j] << "]);\n";
-  o << ind << "}\n";
+  o << ind << "const i64 cap_words = (a.capacity + 31) >> 5;\n";
+  for (size_t j : mo)
+    o << ind << "gx_put_bits(a.out_mask[" << j << "], (i64)pos, total_, "
+      << (slot[j] < 0 ? std::string("gx_ones(total_)") : "vb" + std::to_string(slot[j]) + "_") << ", cap_words);\n";
+  g.masks_ = was;
 }
 
 void emit_filter_writes(std::ostringstream& o, const Gen& g, const Plan& p, const std::vector<int>& pred_ids,
@@ -1292,7 +1361,7 @@ void emit_filter_writes(std::ostringstream& o, const Gen& g, const Plan& p, cons
       const int c = os.col;
       const std::string rt = raw_type(p.schema[c]);
       o << ind << "  if (wr) ((" << rt << "*)a.out_data[" << j << "])[orow] = __ldcs((const " << rt << "*)a.in_data[" << c
-        << "] + a.in_off[" << c << "] + row);\n";
+        << "] + row);\n";
       vexpr = p.nullable[c] ? "gx_valid(a.in_mask[" + std::to_string(c) + "], a.in_off[" + std::to_string(c) + "] + row)"
                             : "true";
     } else {
@@ -1601,8 +1670,8 @@ void emit_fused_tma(std::ostringstream& o, const Gen& g, const Plan& p, const Ti
   for (size_t i = 0; i < L.cols.size(); i++) {
     const int c = L.cols[i];
     const std::string cs = std::to_string(c), w = std::to_string(type_size(p.schema[c]));
-    o << "  const u64 lo" << cs << " = (u64)a.in_data[" << cs << "] + (u64)(a.in_off[" << cs << "] + r0) * " << w
-      << "ull, hi" << cs << " = (u64)a.in_data[" << cs << "] + (u64)(a.in_off[" << cs << "] + r1) * " << w << "ull;\n";
+    o << "  const u64 lo" << cs << " = (u64)a.in_data[" << cs << "] + (u64)r0 * " << w
+      << "ull, hi" << cs << " = (u64)a.in_data[" << cs << "] + (u64)r1 * " << w << "ull;\n";
     if (L.mask_off[i] != UINT32_MAX)
       o << "  const u64 mlo" << cs << " = (u64)(a.in_mask[" << cs << "] + ((a.in_off[" << cs << "] + r0) >> 5)), mhi"
         << cs << " = (u64)(a.in_mask[" << cs << "] + ((a.in_off[" << cs << "] + r1 - 1) >> 5) + 1);\n";
@@ -1701,8 +1770,7 @@ void emit_fused_tma(std::ostringstream& o, const Gen& g, const Plan& p, const Ti
   for (size_t i = 0; i < L.cols.size(); i++) {
     const int c = L.cols[i];
     const std::string cs = std::to_string(c);
-    o << "  const u32 h_" << cs << " = (u32)(((u64)a.in_data[" << cs << "] + (u64)a.in_off[" << cs << "] * "
-      << type_size(p.schema[c]) << "ull) & 15ull);\n";
+    o << "  const u32 h_" << cs << " = (u32)((u64)a.in_data[" << cs << "] & 15ull);\n";
     if (L.mask_off[i] != UINT32_MAX) {
       o << "  const u32 mh_" << cs << " = (u32)((u64)(a.in_mask[" << cs << "] + (a.in_off[" << cs << "] >> 5)) & 15ull);\n";
       o << "  const u32 ms_" << cs << " = (u32)(a.in_off[" << cs << "] & 31);\n";
@@ -2011,8 +2079,8 @@ void emit_staged_filter(std::ostringstream& o, const Gen& g, const Plan& p, cons
       const int w = type_size(p.schema[col]);
       const int cn = 2 * w;  // chunks of this column per word (32 * w / 16)
       o << "            " << (i ? "else " : "") << "if (ck < " << chk + cn << ") gx_cp16(s_buf[s] + GX_T * " << coff[c][i]
-        << " + kw * " << 32 * w << " + (ck - " << chk << ") * 16, (const char*)a.in_data[" << col << "] + (a.in_off["
-        << col << "] + wd * 32) * " << w << " + (ck - " << chk << ") * 16);\n";
+        << " + kw * " << 32 * w << " + (ck - " << chk << ") * 16, (const char*)a.in_data[" << col
+        << "] + (wd * 32) * " << w << " + (ck - " << chk << ") * 16);\n";
       chk += cn;
     }
     o << "          }\n";
@@ -2260,10 +2328,10 @@ std::vector<int> conjunct_columns(const Plan& p, int c) {
 // otherwise idle FP64 pipe takes them.  Conversions (10 to 20 integer
 // instructions), compares with a literal (4) and divisions by a literal or an
 // integer (about 30, against a multiply, two FMAs and the conversions of the
-// operands) are far cheaper on the integer pipes: with them there, against all
-// of them on the FP64 pipe, the order-line plan at 2^27 rows takes 2.43 ms
-// instead of 2.83, its aggregation at 2^26 2.14 instead of 2.45, the deep plan
-// at 2^26 1.70 instead of 1.82.
+// operands) are far cheaper on the integer pipes.  Measured at 2^26 rows of the
+// deep plan: 1.30 ms, 1.42 ms with conversions and 1.47 ms with literal
+// divisions on the FP64 pipe; the order-line plan's two divisions at 2^27 rows
+// cost the same either way (1.88 ms), its aggregation 1.48 ms against 1.64 ms.
 int auto_native_f64_ops() { return kNativeAddSub | kNativeMul; }
 
 std::string generate_kernel(const Plan& p, KernelKind kind, const KernelConfig& cfg_in, const std::string& name) {
@@ -2326,6 +2394,8 @@ std::string generate_kernel(const Plan& p, KernelKind kind, const KernelConfig& 
     o << "  for (i64 w0 = ((i64)blockIdx.x * GX_WARPS + warp) * GX_V; w0 < nwords;"
          " w0 += (i64)gridDim.x * GX_WARPS * GX_V) {\n";
     g.decl(o, ids, "    ");
+    g.masks_ = Gen::Masks::WORDS;
+    g.emit_mask_words(o, ids, {}, "    ");
     // every column load of the warp's words first, then operators and stores
     o << "    #pragma unroll\n    for (int k = 0; k < GX_V; k++) {\n";
     o << "      const i64 row = (w0 + k) * 32 + lane; const bool inr = row < a.n; (void)inr;\n";
@@ -2628,6 +2698,8 @@ std::string generate_agg_kernel(const Plan& p, const AggLayout& L, const KernelC
   o << "    }\n";
   o << "    __syncwarp();\n";
   o << "    const u64 pos = 0ull; (void)pos;\n";
+  g.masks_ = Gen::Masks::KEPT;
+  g.emit_mask_words(o, row_ids, {}, "    ");
   o << "    for (u32 base_ = 0; base_ < total_; base_ += 32u) {\n";
   const std::string in2 = "      ";
   o << in2 << "const u32 t_ = base_ + (u32)lane; const bool act = t_ < total_;\n";

@@ -586,11 +586,7 @@ static void launch(const JitKernel& k, int grid, cudaStream_t s, KernelArgs& arg
 
 static void fill_args_inputs(KernelArgs& a, const std::vector<ColumnView>& cols) {
   std::memset(&a, 0, sizeof a);
-  for (size_t i = 0; i < cols.size(); i++) {
-    a.in_data[i] = cols[i].data;
-    a.in_mask[i] = cols[i].mask;
-    a.in_off[i] = cols[i].offset;
-  }
+  for (size_t i = 0; i < cols.size(); i++) bind_column(a, i, cols[i]);
   a.n = cols.empty() ? 0 : cols[0].size;
 }
 

@@ -27,6 +27,16 @@ struct ColumnView {
 
 std::vector<ColumnView> to_views(const gx_column_view* cols, int n);
 
+// Binds column i of a kernel's argument block: data at the view's first row,
+// validity words from the one that holds the first row's bit, in_off that
+// bit's position (0..31).  With the row offset folded in here, a kernel's
+// column accesses share one index instead of adding an offset per column.
+inline void bind_column(KernelArgs& a, size_t i, const ColumnView& c) {
+  a.in_data[i] = c.data ? (const char*)c.data + c.offset * type_size(c.type) : nullptr;
+  a.in_mask[i] = c.mask ? c.mask + (c.offset >> 5) : nullptr;
+  a.in_off[i] = c.offset & 31;
+}
+
 // stream-ordered device allocation from the device's memory pool; failures
 // raise GX_ERR_OOM (retryable)
 void* dev_alloc(size_t bytes, cudaStream_t s);
