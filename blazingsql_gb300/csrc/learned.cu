@@ -618,6 +618,14 @@ static std::shared_ptr<CompiledPlan> variant(const CompiledPlan& base, int mode,
     // so on request only (GX_STREAM=<slots>)
     const char* st = std::getenv("GX_STREAM");
     c.stream_slots = st && *st ? std::atoi(st) : 0;
+    // The ordered kernel waits on one load per conjunct and word, so resident
+    // warps are what hides it: with outputs that are column copies, few values
+    // are live and 32 registers (64 warps per SM) suffice.  Eight batches of 2^23
+    // rows, two copied outputs: 0.63 ms, 0.66 at 40 registers, 0.72 at 48, 0.83
+    // uncapped (72).  Computed outputs would spill, so they stay uncapped.
+    bool copies = true;
+    for (const auto& os : base.plan().outputs) copies = copies && os.kind == OutSpec::COPY;
+    if (copies && c.max_regs == 0) c.max_regs = 32;
   }
   return std::make_shared<CompiledPlan>(base.plan(), c, mode);
 }
