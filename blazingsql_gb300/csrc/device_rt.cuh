@@ -163,10 +163,19 @@ __device__ __forceinline__ void gx_put_bits(u32* mask, i64 pos, u32 total, u32 b
   // 32 full rounds at an odd position reach a 33rd word
   if (lane == 31 && end > 1024u && w + 1 < cap_words) atomicOr(mask + w + 1, bits >> (32u - sh));
 }
-// lane r's bits for `total` rows that are all valid
-__device__ __forceinline__ u32 gx_ones(u32 total) {
-  const int left = (int)total - (int)(threadIdx.x & 31) * 32;
-  return left >= 32 ? GX_FULL : left <= 0 ? 0u : (1u << left) - 1u;
+// The same for `total` bits that are all ones (any number), by one warp: for
+// outputs that are never NULL a tile's bits need no warp's ballots.
+__device__ __forceinline__ void gx_put_ones(u32* mask, i64 pos, u64 total, i64 cap_words) {
+  const u32 sh = (u32)pos & 31u;
+  const u64 end = sh + total;
+  for (u64 w = threadIdx.x & 31; w * 32u < end; w += 32u) {
+    if ((pos >> 5) + (i64)w >= cap_words) break;
+    u32 v = GX_FULL;
+    if (w == 0) v <<= sh;
+    if ((w + 1u) * 32u > end) v &= (1u << (end & 31u)) - 1u;
+    if (v != GX_FULL) atomicOr(mask + (pos >> 5) + w, v);
+    else mask[(pos >> 5) + w] = v;
+  }
 }
 
 // ---- streaming loads / stores ------------------------------------------------
@@ -338,8 +347,11 @@ __device__ __forceinline__ void gx_st_f32(void* p, i64 i, u64 v) { __stcs((float
 #define GX_ST_PFX (2ull << 62)
 #define GX_ST_VAL ((1ull << 62) - 1ull)
 
-__device__ __forceinline__ void gx_st_release(u64* p, u64 v) {
-  asm volatile("st.release.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
+// A status word carries its flag and its value together, and no other data is
+// published by it, so a relaxed store will do: a release would first wait for
+// the thread's earlier output stores.
+__device__ __forceinline__ void gx_st_status(u64* p, u64 v) {
+  asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
 }
 __device__ __forceinline__ u64 gx_ld_acquire(const u64* p) {
   u64 v;
@@ -356,47 +368,55 @@ __device__ __forceinline__ u64 gx_ld_relaxed(const u64* p) {
 // Exclusive prefix of tile `tile` whose aggregate `agg` is already published
 // (gx_tile_publish); called by one full warp; publishes the tile's inclusive
 // prefix.
-// Each poll reads a window of the 128 preceding status words (4 per lane,
-// lane l holding distances 4l+1 .. 4l+4), sums the aggregates up to the
-// nearest inclusive prefix, and moves 128 tiles further back while none is in
-// the window -- with hundreds of tiles in flight the prefix frontier is that
-// far back, so a wide window saves L2 round trips.  A status word carries its
-// flag and value together, so relaxed loads suffice.  Waits are bounded: after
-// `max_spins` polls without progress it records an error in *err and returns
-// ~0ull (callers then skip their writes); a wait also ends early once *err is
-// set by another tile.
-__device__ __forceinline__ u64 gx_lookback_resolve(u64* status, i64 tile, u64 agg, int* err, u32 max_spins) {
+// Each poll reads a window of the 32 PER preceding status words (load i of lane
+// l at distance 32 i + l + 1, so a load is one coalesced 256-byte request), sums
+// the aggregates up to the nearest inclusive prefix, and moves a window further
+// back while none is in it.  More than a thousand tiles are in flight, and the
+// nearest prefix is far back when tiles resolve slowly: the polls' L2 traffic and
+// registers then set the tile rate of a light filter.  One byte copied per kept
+// row of 2^27: 0.71 ms with 128 words a poll read strided (four times the L2
+// requests), 0.64 ms with 128 coalesced, 0.51 with 64; 256 and 512 are slower
+// (0.70, 0.78).  `known` / `known_incl`: a tile before
+// `tile` whose inclusive prefix the caller already has (its block's previous
+// tile; -1 and 0 when it has none): the walk never reads further back.
+// A status word carries its flag and value together, so relaxed loads suffice.
+// Waits are bounded: after `max_spins` polls without progress it records an
+// error in *err and returns ~0ull (callers then skip their writes); a wait also
+// ends early once *err is set by another tile.
+#define GX_LB_PER 2
+__device__ __forceinline__ u64 gx_lookback_resolve(u64* status, i64 tile, u64 agg, int* err, u32 max_spins,
+                                                   i64 known = -1, u64 known_incl = 0ull) {
   const int lane = threadIdx.x & 31;
   if (tile == 0) return 0ull;  // published as a prefix already
   u64 excl = 0;
   i64 pred = tile - 1;  // distance 1
   u32 spins = 0;
   while (true) {
-    u64 s[4];
+    u64 s[GX_LB_PER];
 #pragma unroll
-    for (int i = 0; i < 4; i++) {
-      const i64 idx = pred - (lane * 4 + i);
-      s[i] = idx >= 0 ? gx_ld_relaxed(status + idx) : GX_ST_PFX;  // before tile 0: prefix 0
+    for (int i = 0; i < GX_LB_PER; i++) {
+      const i64 idx = pred - (i * 32 + lane);
+      // before tile 0: prefix 0
+      s[i] = idx > known ? gx_ld_relaxed(status + idx) : idx == known ? (GX_ST_PFX | known_incl) : GX_ST_PFX;
     }
-    int first_pfx = 4;
+    bool found = false, missing = false;
+    u32 sum = 0u;  // aggregates of one window fit 32 bits
+    u64 prefix = 0ull;
 #pragma unroll
-    for (int i = 3; i >= 0; i--)
-      if ((u32)(s[i] >> 62) == 2u) first_pfx = i;
-    const u32 has_pfx = __ballot_sync(GX_FULL, first_pfx < 4);
-    const int pl = has_pfx ? __ffs(has_pfx) - 1 : 0;
-    const int pfx_i = __shfl_sync(GX_FULL, first_pfx, pl);
-    // entries at window positions <= last (4 lane + i) are needed
-    const int last = has_pfx ? pl * 4 + pfx_i : 127;
-    bool missing = false;
-    u64 v = 0;
-#pragma unroll
-    for (int i = 0; i < 4; i++) {
-      if (lane * 4 + i <= last) {
-        if ((u32)(s[i] >> 62) == 0u) missing = true;
-        v += s[i] & GX_ST_VAL;
+    for (int i = 0; i < GX_LB_PER; i++) {
+      if (!found) {
+        const u32 pfx = __ballot_sync(GX_FULL, (u32)(s[i] >> 62) == 2u);
+        const u32 none = __ballot_sync(GX_FULL, (u32)(s[i] >> 62) == 0u);
+        const u32 before = pfx ? (pfx & (0u - pfx)) - 1u : GX_FULL;  // lanes nearer than the prefix
+        missing = missing || (none & before) != 0u;
+        if ((before >> lane) & 1u) sum += (u32)s[i];
+        if (pfx) {
+          found = true;
+          prefix = __shfl_sync(GX_FULL, s[i], __ffs(pfx) - 1) & GX_ST_VAL;
+        }
       }
     }
-    if (__any_sync(GX_FULL, missing)) {
+    if (missing) {
       if (++spins > max_spins) {
         if (lane == 0) atomicExch(err, 1);
         return ~0ull;
@@ -406,13 +426,11 @@ __device__ __forceinline__ u64 gx_lookback_resolve(u64* status, i64 tile, u64 ag
       __nanosleep(32);
       continue;
     }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(GX_FULL, v, o);
-    excl += v;
-    if (has_pfx) break;
-    pred -= 128;
+    excl += prefix + (u64)__reduce_add_sync(GX_FULL, sum);
+    if (found) break;
+    pred -= 32 * GX_LB_PER;
   }
-  if (lane == 0) gx_st_release(status + tile, GX_ST_PFX | (excl + agg));
+  if (lane == 0) gx_st_status(status + tile, GX_ST_PFX | (excl + agg));
   return excl;
 }
 
@@ -469,7 +487,7 @@ __device__ __forceinline__ u64 gx_lookback_wide(u64* status, i64 tile, u64 agg, 
     if (has_pfx) break;
     pred -= 32 * PER;
   }
-  if (lane == 0) gx_st_release(status + tile, GX_ST_PFX | (excl + agg));
+  if (lane == 0) gx_st_status(status + tile, GX_ST_PFX | (excl + agg));
   return excl;
 }
 
@@ -522,9 +540,29 @@ __device__ __forceinline__ bool gx_lookback_poll(u64* status, i64 tile, u64 agg,
     if (has_pfx) break;
     pr -= 128;
   }
-  if (lane == 0) gx_st_release(status + tile, GX_ST_PFX | (ex + agg));
+  if (lane == 0) gx_st_status(status + tile, GX_ST_PFX | (ex + agg));
   *excl = ex;
   return true;
+}
+
+// The tile pipeline's count hand-over on named barrier 2: the first warp waits
+// until every warp of the block has written its count to shared memory, the
+// others go on at once.
+__device__ __forceinline__ void gx_bar_counts(int warp, int nw) {
+  if (nw == 1) __syncwarp();
+  else if (warp == 0) asm volatile("bar.sync 2, %0;" ::"r"(nw * 32) : "memory");
+  else asm volatile("bar.arrive 2, %0;" ::"r"(nw * 32) : "memory");
+}
+
+// The batch that holds global tile gt, at or after batch b (tile_base
+// ascending; a warp looks at 32 batches per step).
+__device__ __forceinline__ int gx_find_batch(const long long* __restrict__ tile_base, int b, int nbatch, long long gt) {
+  while (true) {
+    const int i = b + 1 + (int)(threadIdx.x & 31);
+    const int n = __popc(__ballot_sync(GX_FULL, i < nbatch && __ldg(tile_base + i) <= gt));
+    b += n;
+    if (n < 32) return b;
+  }
 }
 
 // Publishes a tile's aggregate (tile 0: its inclusive prefix) from the
@@ -542,14 +580,14 @@ __device__ __forceinline__ u64 gx_tile_publish(u64* status, i64 tile, const u32*
   }
   const u64 total = __shfl_sync(GX_FULL, incl, 31);
   if (lane < nw) off[lane] = incl - c;
-  if (lane == 0) gx_st_release(status + tile, (tile == 0 ? GX_ST_PFX : GX_ST_AGG) | total);
+  if (lane == 0) gx_st_status(status + tile, (tile == 0 ? GX_ST_PFX : GX_ST_AGG) | total);
   return total;
 }
 
 // Publish + resolve in one step (tile loops without a pipeline).
 __device__ __forceinline__ u64 gx_lookback(u64* status, i64 tile, u64 agg, int* err, u32 max_spins) {
   const int lane = threadIdx.x & 31;
-  if (lane == 0) gx_st_release(status + tile, (tile == 0 ? GX_ST_PFX : GX_ST_AGG) | agg);
+  if (lane == 0) gx_st_status(status + tile, (tile == 0 ? GX_ST_PFX : GX_ST_AGG) | agg);
   return gx_lookback_resolve(status, tile, agg, err, max_spins);
 }
 

@@ -411,7 +411,10 @@ class Gen {
   // the load of a column's element at `row` (data pointers start at the batch's first row)
   std::string load_call(int c) const {
     std::string fn = emu() ? load_fn_emu(p_.schema[c]) : load_fn(p_.schema[c]);
-    if (reread_cols_.count(c)) fn = "gx_ldg_" + fn.substr(6);  // gx_ld_X -> gx_ldg_X
+    // a kept-row round starts and ends inside a sector that its neighbours read
+    // too, so it loads with the default policy (order-line plan 2^27: 1.75 ms
+    // against 1.89 with evict-first loads)
+    if (reread_cols_.count(c) || masks_ == Masks::KEPT) fn = "gx_ldg_" + fn.substr(6);  // gx_ld_X -> gx_ldg_X
     return fn + "(a.in_data[" + std::to_string(c) + "], row)";
   }
   // where a row's validity bit is read from
@@ -1165,10 +1168,22 @@ std::vector<size_t> masked_outputs(const Plan& p) {
   return v;
 }
 
+// The warp's kept rows in order, from its keep masks `bal`: offsets from its
+// first row, listed in `list` (GX_V * 32 entries of shared memory) by kept rank;
+// declares and counts `total`.
+void emit_kept_list(std::ostringstream& o, const std::string& bal, const std::string& list, const std::string& total,
+                    const std::string& ind) {
+  o << ind << "#pragma unroll\n" << ind << "for (int kk = 0; kk < GX_V; kk++) {\n";
+  o << ind << "  if ((" << bal << "[kk] >> lane) & 1u) " << list << "[" << total << " + __popc(" << bal
+    << "[kk] & ((1u << lane) - 1u))] = (unsigned short)(kk * 32 + lane);\n";
+  o << ind << "  " << total << " += __popc(" << bal << "[kk]);\n";
+  o << ind << "}\n";
+}
+
 // statements mapping kept rank t_ of the warp (0 <= t_ < total_) to its row
-// through the warp's kept-row list in shared memory
+// through the warp's kept-row list kl_ in shared memory
 void emit_rank_to_row(std::ostringstream& o, const std::string& ind) {
-  o << ind << "const u32 kp_ = act ? (u32)s_kept_[warp][t_] : 0u; const i64 row = w0 * 32 + kp_; const bool inr = act; (void)inr;\n";
+  o << ind << "const u32 kp_ = act ? (u32)kl_[t_] : 0u; const i64 row = w0 * 32 + kp_; const bool inr = act; (void)inr;\n";
   o << ind << "const i64 orow = (i64)pos + (i64)t_; (void)orow;\n";
   o << ind << "const int k = 0;\n";
 }
@@ -1210,7 +1225,10 @@ void emit_row_nodes(std::ostringstream& o, const Gen& g, const Plan& p, const st
 // lane's store per mask and round.  340 -> 285 instructions, call time at 2^27
 // rows 2.43 -> 2.08 ms; deep plan 2^26 1.70 -> 1.47; process_filter of six
 // columns 2^23 0.346 -> 0.274.
-void emit_filter_writes_dense(std::ostringstream& o, const Gen& g, const Plan& p, const std::string& ind) {
+// The list kl_ of the warp's total_ kept rows is made here from bal[], unless the
+// caller has made it (`listed`).
+void emit_filter_writes_dense(std::ostringstream& o, const Gen& g, const Plan& p, const std::string& ind,
+                              bool listed = false) {
   const std::vector<int> roots = g.output_roots();
   const std::vector<Gen::Lazy> lz = g.lazy_branches(roots);
   std::map<int, int> lz_root;
@@ -1228,14 +1246,13 @@ void emit_filter_writes_dense(std::ostringstream& o, const Gen& g, const Plan& p
       if (os.kind == OutSpec::COPY) copied.push_back(os.col);
     g.emit_mask_words(o, g.cone(roots), copied, ind);
   }
-  // the warp's kept rows in order: offsets from its first row, by kept rank
-  o << ind << "__shared__ unsigned short s_kept_[GX_WARPS][GX_V * 32];\n";
-  o << ind << "u32 total_ = 0u;\n";
-  o << ind << "#pragma unroll\n" << ind << "for (int kk = 0; kk < GX_V; kk++) {\n";
-  o << ind << "  if ((bal[kk] >> lane) & 1u) s_kept_[warp][total_ + __popc(bal[kk] & ((1u << lane) - 1u))] = (unsigned short)(kk * 32 + lane);\n";
-  o << ind << "  total_ += __popc(bal[kk]);\n";
-  o << ind << "}\n";
-  o << ind << "__syncwarp();\n";
+  if (!listed) {
+    o << ind << "__shared__ unsigned short s_kept_[GX_WARPS][GX_V * 32];\n";
+    o << ind << "unsigned short* const kl_ = s_kept_[warp];\n";
+    o << ind << "u32 total_ = 0u;\n";
+    emit_kept_list(o, "bal", "kl_", "total_", ind);
+    o << ind << "__syncwarp();\n";
+  }
   if (!lz.empty()) {
     const int nl = (int)lz.size();
     o << ind << "__shared__ u64 s_lzb_[" << nl << "][GX_WARPS][GX_V * 32];\n";
@@ -1305,8 +1322,8 @@ void emit_filter_writes_dense(std::ostringstream& o, const Gen& g, const Plan& p
     if (p.outputs[j].kind != OutSpec::COPY) continue;
     const int c = p.outputs[j].col;
     const std::string rt = raw_type(p.schema[c]);
-    o << in2 << "const " << rt << " r" << j << "_ = act ? " << (g.reread_cols_.count(c) ? "__ldg" : "__ldcs") << "((const "
-      << rt << "*)a.in_data[" << c << "] + row) : (" << rt << ")0;\n";
+    o << in2 << "const " << rt << " r" << j << "_ = act ? __ldg((const " << rt << "*)a.in_data[" << c << "] + row) : ("
+      << rt << ")0;\n";
   }
   emit_row_nodes(o, g, p, proj, lz_root, in2);
   o << in2 << "const bool wr = t_ < wmax_;\n";
@@ -1319,9 +1336,29 @@ void emit_filter_writes_dense(std::ostringstream& o, const Gen& g, const Plan& p
   o << ind << "}\n";
   o << ind << "__syncwarp();\n";  // the kept-row list and branch results are rewritten by the next tile
   o << ind << "const i64 cap_words = (a.capacity + 31) >> 5;\n";
-  for (size_t j : mo)
-    o << ind << "gx_put_bits(a.out_mask[" << j << "], (i64)pos, total_, "
-      << (slot[j] < 0 ? std::string("gx_ones(total_)") : "vb" + std::to_string(slot[j]) + "_") << ", cap_words);\n";
+  for (size_t j : mo) {
+    if (slot[j] >= 0)
+      o << ind << "gx_put_bits(a.out_mask[" << j << "], (i64)pos, total_, vb" << slot[j] << "_, cap_words);\n";
+    else if (!listed)  // else the block writes its tile's (emit_tile_ones)
+      o << ind << "gx_put_ones(a.out_mask[" << j << "], (i64)pos, total_, cap_words);\n";
+  }
+  g.masks_ = was;
+}
+
+// The validity bits of the outputs that are never NULL, for a whole tile: its
+// rows' bits are all ones from the tile's base on, so the block's warps share
+// the masks out, one warp per mask.
+void emit_tile_ones(std::ostringstream& o, const Gen& g, const Plan& p, const std::string& base, const std::string& total,
+                    const std::string& ind) {
+  const Gen::Masks was = g.masks_;
+  g.masks_ = Gen::Masks::KEPT;
+  int i = 0;
+  for (size_t j : masked_outputs(p)) {
+    const OutSpec& os = p.outputs[j];
+    if (os.kind == OutSpec::COPY ? g.masked(os.col) : !g.never_null(os.node)) continue;
+    o << ind << "if (warp == " << i++ << " % GX_WARPS) gx_put_ones(a.out_mask[" << j << "], (i64)" << base << ", " << total
+      << ", (a.capacity + 31) >> 5);\n";
+  }
   g.masks_ = was;
 }
 
@@ -1380,13 +1417,19 @@ void emit_filter_writes(std::ostringstream& o, const Gen& g, const Plan& p, cons
 }
 
 // Fused single-pass filter (dense projections) as a two-stage tile pipeline:
-// a block claims tile t+1 and evaluates its predicate before it resolves tile
-// t's output offset by look-back, so the look-back of t waits on tiles that
-// had a whole tile's time to publish, and the next tile's loads are in flight
-// meanwhile.  Tile t's keep masks stay in registers between the stages (dense
-// projections recompute outputs from the gathered rows).  A claimed tile's
-// aggregate is published before the block waits on anything, and a tile's
-// look-back only needs earlier tiles, so the pipeline cannot deadlock.
+// a block evaluates tile t+1's predicate before it resolves tile t's output
+// offset by look-back, so the look-back of t waits on tiles that had a whole
+// tile's time to publish, and the next tile's loads are in flight meanwhile.
+// Between the stages tile t is its warps' kept-row lists in shared memory
+// (dense projections recompute outputs from the gathered rows).
+//
+// The block is bound by what its warps wait for, so they wait for little: the
+// ticket of tile t+2 is drawn while t+1 is evaluated (an atomic's round trip to
+// L2 otherwise starts every tile), warps other than the first only announce
+// their counts (bar.arrive) and go on, and meet the first one once per tile,
+// when the offset is known.  No deadlock: the block that holds the first
+// unpublished tile waits at most for earlier tiles, all of them published, so
+// it comes to evaluate and publish it.
 void emit_fused_pipelined(std::ostringstream& o, const Gen& g, const Plan& p, const std::vector<int>& pred_ids) {
   // with conj_stats (fixed order, every conjunct evaluated for every row): each
   // conjunct's passing rows, counted per warp in registers and added to
@@ -1406,60 +1449,66 @@ void emit_fused_pipelined(std::ostringstream& o, const Gen& g, const Plan& p, co
   o << "  __shared__ unsigned long long s_claim;\n";
   o << "  __shared__ u32 s_cnt[2][GX_WARPS];\n";
   o << "  __shared__ u64 s_off[2][GX_WARPS];\n";
-  o << "  __shared__ u64 s_base;\n";
+  o << "  __shared__ u64 s_base, s_total;\n";
+  o << "  __shared__ unsigned short s_kept_[2][GX_WARPS][GX_V * 32];\n";
   o << "  const i64 ntiles = (nwords + GX_TILE_WORDS - 1) / GX_TILE_WORDS;\n";
   o << "  if (threadIdx.x == 0) s_claim = atomicAdd(a.tile_counter, 1ull);\n";
   o << "  __syncthreads();\n";
   o << "  i64 tile = (i64)s_claim;\n";
   o << "  if (tile >= ntiles) return;\n";
-  o << "  u32 bal[GX_V]; u32 wcnt = 0u; int par = 0; u64 ptotal = 0ull;\n";
+  o << "  __syncthreads();\n";  // s_claim is rewritten below
+  o << "  u32 wcnt = 0u; int par = 0; u64 ptotal = 0ull; unsigned long long ahead_ = 0ull;\n";
+  o << "  i64 known_ = -1; u64 known_incl_ = 0ull;\n";  // the block's last resolved tile and its inclusive prefix
+  o << "  if (threadIdx.x == 0) ahead_ = atomicAdd(a.tile_counter, 1ull);\n";
   o << "  {\n";
   o << "    const i64 w0 = tile * GX_TILE_WORDS + (i64)warp * GX_V;\n";
-  g.decl(o, pred_ids, "    ");
-  g.emit_predicate(o, "    ");
-  count_conjuncts("    ");
-  o << "    #pragma unroll\n    for (int k = 0; k < GX_V; k++) { bal[k] = __ballot_sync(GX_FULL, alive[k]); wcnt += __popc(bal[k]); }\n";
-  o << "    if (lane == 0) s_cnt[0][warp] = wcnt;\n";
+  auto predicate = [&](const std::string& buf, const std::string& cnt, const std::string& ind) {
+    g.decl(o, pred_ids, ind);
+    g.emit_predicate(o, ind);
+    count_conjuncts(ind);
+    o << ind << "u32 bal[GX_V];\n";
+    o << ind << "#pragma unroll\n" << ind << "for (int k = 0; k < GX_V; k++) bal[k] = __ballot_sync(GX_FULL, alive[k]);\n";
+    emit_kept_list(o, "bal", "s_kept_[" + buf + "][warp]", cnt, ind);
+    o << ind << "if (lane == 0) s_cnt[" << buf << "][warp] = " << cnt << ";\n";
+  };
+  predicate("0", "wcnt", "    ");
   o << "  }\n";
+  o << "  if (threadIdx.x == 0) s_claim = ahead_;\n";
   o << "  __syncthreads();\n";
   o << "  if (warp == 0) ptotal = gx_tile_publish(a.tile_status, tile, s_cnt[0], s_off[0], GX_WARPS);\n";
   o << "  while (true) {\n";
-  o << "    if (threadIdx.x == 0) s_claim = atomicAdd(a.tile_counter, 1ull);\n";
-  o << "    __syncthreads();\n";
   o << "    const i64 next = (i64)s_claim;\n";
+  o << "    if (threadIdx.x == 0 && next < ntiles) ahead_ = atomicAdd(a.tile_counter, 1ull);\n";
   o << "    const int npar = par ^ 1;\n";
-  o << "    u32 nbal[GX_V]; u32 nwcnt = 0u;\n";
-  o << "    #pragma unroll\n    for (int k = 0; k < GX_V; k++) nbal[k] = 0u;\n";
+  o << "    u32 nwcnt = 0u;\n";
   o << "    if (next < ntiles) {\n";
   o << "      const i64 w0 = next * GX_TILE_WORDS + (i64)warp * GX_V;\n";
-  g.decl(o, pred_ids, "      ");
-  g.emit_predicate(o, "      ");
-  count_conjuncts("      ");
-  o << "      #pragma unroll\n      for (int k = 0; k < GX_V; k++) { nbal[k] = __ballot_sync(GX_FULL, alive[k]); nwcnt += __popc(nbal[k]); }\n";
-  o << "      if (lane == 0) s_cnt[npar][warp] = nwcnt;\n";
+  predicate("npar", "nwcnt", "      ");
   o << "    }\n";
-  o << "    __syncthreads();\n";
+  o << "    gx_bar_counts(warp, GX_WARPS);\n";  // the first warp waits for every warp's count
   o << "    if (warp == 0) {\n";
   o << "      u64 ntotal = 0ull;\n";
   o << "      if (next < ntiles) ntotal = gx_tile_publish(a.tile_status, next, s_cnt[npar], s_off[npar], GX_WARPS);\n";
-  o << "      const u64 excl = gx_lookback_resolve(a.tile_status, tile, ptotal, a.err, GX_SPINS);\n";
+  o << "      const u64 excl = gx_lookback_resolve(a.tile_status, tile, ptotal, a.err, GX_SPINS, known_, known_incl_);\n";
   o << "      if (lane == 0) {\n";
-  o << "        s_base = excl;\n";
+  o << "        s_base = excl; s_total = ptotal; s_claim = ahead_;\n";
   o << "        if (tile == ntiles - 1 && excl != ~0ull) *a.out_count = excl + ptotal;\n";
   o << "      }\n";
+  o << "      known_ = tile; known_incl_ = excl + ptotal;\n";
   o << "      ptotal = ntotal;\n";
   o << "    }\n";
   o << "    __syncthreads();\n";
   o << "    const u64 base_t = s_base;\n";
   o << "    if (base_t == ~0ull) break;\n";  // look-back gave up: error already recorded
+  emit_tile_ones(o, g, p, "base_t", "s_total", "    ");
   o << "    if (wcnt != 0u) {\n";
   o << "      u64 pos = base_t + s_off[par][warp];\n";
   o << "      const i64 w0 = tile * GX_TILE_WORDS + (i64)warp * GX_V;\n";
-  emit_filter_writes_dense(o, g, p, "      ");
+  o << "      const unsigned short* const kl_ = s_kept_[par][warp]; const u32 total_ = wcnt;\n";
+  emit_filter_writes_dense(o, g, p, "      ", true);
   o << "    }\n";
   o << "    if (next >= ntiles) break;\n";
   o << "    tile = next; par = npar; wcnt = nwcnt;\n";
-  o << "    #pragma unroll\n    for (int k = 0; k < GX_V; k++) bal[k] = nbal[k];\n";
   o << "  }\n";
   if (stats) {
     o << "  if (lane == 0) {\n";
@@ -1823,7 +1872,7 @@ void emit_fused_tma(std::ostringstream& o, const Gen& g, const Plan& p, const Ti
   o << "    u32 tot_ = 0u, woff = 0u;\n";
   o << "    if (tile >= 0) woff = gx_block_excl(s_cnt_[vp], GX_WARPS, &tot_, warp);\n";
   o << "    if (warp == 0 && lane == 0) {\n";
-  o << "      if (tile >= 0) gx_st_release(a.tile_status + tile, (tile == 0 ? GX_ST_PFX : GX_ST_AGG) | (u64)tot_);\n";
+  o << "      if (tile >= 0) gx_st_status(a.tile_status + tile, (tile == 0 ? GX_ST_PFX : GX_ST_AGG) | (u64)tot_);\n";
   o << "      s_rtile_[rr] = tile; s_ragg_[rr] = (u64)tot_;\n";
   o << "      gx_mbar_arrive(&s_counted_[rr]);\n";
   o << "    }\n";
@@ -1920,7 +1969,13 @@ void emit_fused_batched(std::ostringstream& o, const Gen& g, const Plan& p, cons
   o << "  __shared__ unsigned long long s_claim;\n";
   o << "  __shared__ u32 s_cnt[2][GX_WARPS];\n";
   o << "  __shared__ u64 s_off[2][GX_WARPS];\n";
-  o << "  __shared__ u64 s_base;\n";
+  o << "  __shared__ u64 s_base, s_total;\n";
+  o << "  __shared__ unsigned short s_kept_[2][GX_WARPS][GX_V * 32];\n";
+  // the batch of global tile gt, at or after batch b
+  auto find = [&](const std::string& b, const std::string& gt, const std::string& ind) {
+    if (streaming) o << ind << "while (" << b << " + 1 < nbatch && tile_base[" << b << " + 1] <= " << gt << ") " << b << "++;\n";
+    else o << ind << b << " = gx_find_batch(tile_base, " << b << ", nbatch, " << gt << ");\n";
+  };
   if (streaming) {
     o << "  if (threadIdx.x == 0) s_claim = (unsigned long long)claim_();\n";
     o << "  __syncthreads();\n";
@@ -1932,66 +1987,82 @@ void emit_fused_batched(std::ostringstream& o, const Gen& g, const Plan& p, cons
     o << "  const i64 gt0 = (i64)s_claim;\n";
     o << "  if (gt0 >= total_tiles) return;\n";
   }
+  o << "  __syncthreads();\n";  // s_claim is rewritten below
+  // the ticket after next is drawn ahead (as emit_fused_pipelined), but for a
+  // queue that the host extends: there a claim may wait for the host
+  if (!streaming) {
+    o << "  unsigned long long ahead_ = 0ull;\n";
+    o << "  if (threadIdx.x == 0) ahead_ = atomicAdd(&hdr->tile_counter, 1ull);\n";
+  }
   o << "  int pb = 0;\n";
-  o << "  while (pb + 1 < nbatch && tile_base[pb + 1] <= gt0) pb++;\n";
+  find("pb", "gt0", "  ");
   o << "  i64 tile = gt0 - tile_base[pb];\n";
-  o << "  u32 bal[GX_V]; u32 wcnt = 0u; int par = 0; u64 ptotal = 0ull;\n";
+  o << "  u32 wcnt = 0u; int par = 0; u64 ptotal = 0ull;\n";
+  o << "  i64 known_ = -1; u64 known_incl_ = 0ull;\n";  // the block's last resolved tile of this batch
+  auto predicate = [&](const std::string& buf, const std::string& cnt, const std::string& ind) {
+    g.decl(o, pred_ids, ind);
+    g.emit_predicate(o, ind);
+    o << ind << "u32 bal[GX_V];\n";
+    o << ind << "#pragma unroll\n" << ind << "for (int k = 0; k < GX_V; k++) bal[k] = __ballot_sync(GX_FULL, alive[k]);\n";
+    emit_kept_list(o, "bal", "s_kept_[" + buf + "][warp]", cnt, ind);
+    o << ind << "if (lane == 0) s_cnt[" << buf << "][warp] = " << cnt << ";\n";
+  };
   o << "  {\n";
   o << "    const GxArgs& a = GX_BATCH(pb);\n";
   o << "    const i64 w0 = tile * GX_TILE_WORDS + (i64)warp * GX_V;\n";
-  g.decl(o, pred_ids, "    ");
-  g.emit_predicate(o, "    ");
-  o << "    #pragma unroll\n    for (int k = 0; k < GX_V; k++) { bal[k] = __ballot_sync(GX_FULL, alive[k]); wcnt += __popc(bal[k]); }\n";
-  o << "    if (lane == 0) s_cnt[0][warp] = wcnt;\n";
+  predicate("0", "wcnt", "    ");
   o << "  }\n";
+  if (!streaming) o << "  if (threadIdx.x == 0) s_claim = ahead_;\n";
   o << "  __syncthreads();\n";
   o << "  if (warp == 0) ptotal = gx_tile_publish(GX_BATCH(pb).tile_status, tile, s_cnt[0], s_off[0], GX_WARPS);\n";
   o << "  while (true) {\n";
-  if (streaming) o << "    if (threadIdx.x == 0) s_claim = (unsigned long long)claim_();\n";
-  else o << "    if (threadIdx.x == 0) s_claim = atomicAdd(&hdr->tile_counter, 1ull);\n";
-  o << "    __syncthreads();\n";
+  if (streaming) {
+    o << "    if (threadIdx.x == 0) s_claim = (unsigned long long)claim_();\n";
+    o << "    __syncthreads();\n";
+  }
   o << "    const i64 ngt = (i64)s_claim;\n";
   o << "    int nb = pb; i64 next = -1;\n";
   o << "    if (" << (streaming ? "ngt >= 0" : "ngt < total_tiles") << ") {\n";
-  o << "      while (nb + 1 < nbatch && tile_base[nb + 1] <= ngt) nb++;\n";
+  if (!streaming) o << "      if (threadIdx.x == 0) ahead_ = atomicAdd(&hdr->tile_counter, 1ull);\n";
+  find("nb", "ngt", "      ");
   o << "      next = ngt - tile_base[nb];\n";
   o << "    }\n";
   o << "    const int npar = par ^ 1;\n";
-  o << "    u32 nbal[GX_V]; u32 nwcnt = 0u;\n";
-  o << "    #pragma unroll\n    for (int k = 0; k < GX_V; k++) nbal[k] = 0u;\n";
+  o << "    u32 nwcnt = 0u;\n";
   o << "    if (next >= 0) {\n";
   o << "      const GxArgs& a = GX_BATCH(nb);\n";
   o << "      const i64 w0 = next * GX_TILE_WORDS + (i64)warp * GX_V;\n";
-  g.decl(o, pred_ids, "      ");
-  g.emit_predicate(o, "      ");
-  o << "      #pragma unroll\n      for (int k = 0; k < GX_V; k++) { nbal[k] = __ballot_sync(GX_FULL, alive[k]); nwcnt += __popc(nbal[k]); }\n";
-  o << "      if (lane == 0) s_cnt[npar][warp] = nwcnt;\n";
+  predicate("npar", "nwcnt", "      ");
   o << "    }\n";
-  o << "    __syncthreads();\n";
+  o << "    gx_bar_counts(warp, GX_WARPS);\n";
   o << "    if (warp == 0) {\n";
   o << "      u64 ntotal = 0ull;\n";
   o << "      if (next >= 0) ntotal = gx_tile_publish(GX_BATCH(nb).tile_status, next, s_cnt[npar], s_off[npar], GX_WARPS);\n";
   o << "      const GxArgs& a = GX_BATCH(pb);\n";
   o << "      const i64 ntiles = (((a.n + 31) >> 5) + GX_TILE_WORDS - 1) / GX_TILE_WORDS;\n";
-  o << "      const u64 excl = gx_lookback_resolve(a.tile_status, tile, ptotal, a.err, GX_SPINS);\n";
+  o << "      const u64 excl = gx_lookback_resolve(a.tile_status, tile, ptotal, a.err, GX_SPINS, known_, known_incl_);\n";
   o << "      if (lane == 0) {\n";
-  o << "        s_base = excl;\n";
+  o << "        s_base = excl; s_total = ptotal;" << (streaming ? "" : " s_claim = ahead_;") << "\n";
   o << "        if (tile == ntiles - 1 && excl != ~0ull) *a.out_count = excl + ptotal;\n";
   o << "      }\n";
+  o << "      known_ = nb == pb ? tile : -1; known_incl_ = nb == pb ? excl + ptotal : 0ull;\n";
   o << "      ptotal = ntotal;\n";
   o << "    }\n";
   o << "    __syncthreads();\n";
   o << "    const u64 base_t = s_base;\n";
   o << "    if (base_t == ~0ull) break;\n";  // look-back gave up: error already recorded
+  o << "    {\n      const GxArgs& a = GX_BATCH(pb);\n";
+  emit_tile_ones(o, g, p, "base_t", "s_total", "      ");
+  o << "    }\n";
   o << "    if (wcnt != 0u) {\n";
   o << "      const GxArgs& a = GX_BATCH(pb);\n";
   o << "      u64 pos = base_t + s_off[par][warp];\n";
   o << "      const i64 w0 = tile * GX_TILE_WORDS + (i64)warp * GX_V;\n";
-  emit_filter_writes_dense(o, g, p, "      ");
+  o << "      const unsigned short* const kl_ = s_kept_[par][warp]; const u32 total_ = wcnt;\n";
+  emit_filter_writes_dense(o, g, p, "      ", true);
   o << "    }\n";
   o << "    if (next < 0) break;\n";
   o << "    tile = next; pb = nb; par = npar; wcnt = nwcnt;\n";
-  o << "    #pragma unroll\n    for (int k = 0; k < GX_V; k++) bal[k] = nbal[k];\n";
   o << "  }\n";
   o << "}\n";
 }
@@ -2691,11 +2762,8 @@ std::string generate_agg_kernel(const Plan& p, const AggLayout& L, const KernelC
   o << "      #pragma unroll\n      for (int k = 0; k < GX_V; k++) bal[k] = __ballot_sync(GX_FULL, alive[k]);\n";
   o << "    }\n";
   o << "    u32 total_ = 0u;\n";
-  o << "    #pragma unroll\n    for (int kk = 0; kk < GX_V; kk++) {\n";
-  o << "      if ((bal[kk] >> lane) & 1u) s_kept_[warp][total_ + __popc(bal[kk] & ((1u << lane) - 1u))] = "
-       "(unsigned short)(kk * 32 + lane);\n";
-  o << "      total_ += __popc(bal[kk]);\n";
-  o << "    }\n";
+  o << "    unsigned short* const kl_ = s_kept_[warp];\n";
+  emit_kept_list(o, "bal", "kl_", "total_", "    ");
   o << "    __syncwarp();\n";
   o << "    const u64 pos = 0ull; (void)pos;\n";
   g.masks_ = Gen::Masks::KEPT;

@@ -434,18 +434,28 @@ static const char* kind_name(KernelKind k) {
 
 // Candidate block shapes (warps x words, register cap) of a tuned single-pass
 // filter: the first is used until the others have been measured.  Measured on
-// GB300: the deep C2 plan is fastest at 4 x 8, the order-line C5 plan at 1 x 16
-// (no block barrier between warps), the light C1 plan at 4 x 8 held to 40
-// registers (more resident warps for a latency-bound pass: 0.179 ms against
-// 0.191 at 1 x 16 and 0.220 at 4 x 8 uncapped, 2^24 rows).
-static const CompiledPlan::Shape kShapes[] = {{4, 8, 0}, {1, 16, 0}, {2, 8, 0}, {4, 8, 40}};
+// GB300 (kernel us; light C1 plan 2^24 rows / deep C2 2^26 / order-line C5 2^27 /
+// process_filter of six columns 2^23): 4 x 8 137 / 1258 / 1733 / 104, 4 x 8 held
+// to 48 registers (more resident warps for a plan that waits on loads) 127 /
+// 1434 / 1676 / 142, 2 x 8 137 / 1252 / 1864 / 109, 8 x 8 at 48 registers 125 /
+// 1625 / 1692 / 137.  Not worth a trial: 1 x 16 150 / 1706 / 1797 / 114, 4 x 4
+// 151 / 1836 / 1809 / 105, 4 x 16 157 / 1883 / 1860 / 129, 40 registers.
+static const CompiledPlan::Shape kShapes[] = {{4, 8, 0}, {4, 8, 48}, {2, 8, 0}, {8, 8, 48}};
 static constexpr int kNumShapes = 4;
+// Small calls leave most of the chip idle, so a tile's latency counts: 8 x 4 has
+// half the serial words per warp of 4 x 8 for the same tile of 1024 rows.
+// Kernel us at 8 x 4 / 4 x 8: order-line plan 10.3 / 13.1 at 1031 rows, 10.4 /
+// 12.1 at 100,003, 24.0 / 32.2 at 1,000,003; from 4,000,000 rows on the large
+// shapes win (69.9 / 66.2; deep plan 133 / 108).
+static constexpr CompiledPlan::Shape kSmallShape{8, 4, 0};
+static constexpr int64_t kSmallRows = int64_t(1) << 21;
 
 // The first large call runs the first candidate unmeasured (it pays the
 // first touches of fresh output memory), the next ones measure each candidate.
 CompiledPlan::Shape CompiledPlan::filter_shape(int64_t n, int* explore) const {
   *explore = -1;
   if (!cfg_.tune_shape) return {cfg_.warps, cfg_.words, 0};
+  if (n < kSmallRows) return kSmallShape;
   std::lock_guard<std::mutex> g(tmu_);
   if (chosen_ >= 0) return kShapes[chosen_];
   if (cand_ms_.empty()) cand_ms_.assign(kNumShapes, -1.f);
