@@ -340,6 +340,9 @@ __device__ __forceinline__ void gx_st_32(void* p, i64 i, u64 v) { __stcs((int*)p
 __device__ __forceinline__ void gx_st_64(void* p, i64 i, u64 v) { __stcs((long long*)p + i, (long long)v); }
 __device__ __forceinline__ void gx_st_f32(void* p, i64 i, u64 v) { __stcs((float*)p + i, (float)gx_D(v)); }
 
+// records an error code (the word may lie in mapped host memory, so a plain store)
+__device__ __forceinline__ void gx_set_err(int* err, int code) { *(volatile int*)err = code; }
+
 // ---- decoupled look-back (single-pass stable compaction) --------------------
 // tile status word: bits 62..63 flag (0 none, 1 aggregate, 2 inclusive prefix),
 // bits 0..61 value.
@@ -418,7 +421,7 @@ __device__ __forceinline__ u64 gx_lookback_resolve(u64* status, i64 tile, u64 ag
     }
     if (missing) {
       if (++spins > max_spins) {
-        if (lane == 0) atomicExch(err, 1);
+        if (lane == 0) gx_set_err(err, 1);
         return ~0ull;
       }
       // another tile already gave up: its successors never complete, stop now
@@ -474,7 +477,7 @@ __device__ __forceinline__ u64 gx_lookback_wide(u64* status, i64 tile, u64 agg, 
     }
     if (__any_sync(GX_FULL, missing)) {
       if (++spins > max_spins) {
-        if (lane == 0) atomicExch(err, 1);
+        if (lane == 0) gx_set_err(err, 1);
         return ~0ull;
       }
       if ((spins & 255u) == 0u && *(volatile int*)err != 0) return ~0ull;

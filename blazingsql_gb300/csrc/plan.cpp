@@ -1761,7 +1761,7 @@ void emit_fused_tma(std::ostringstream& o, const Gen& g, const Plan& p, const Ti
   }
   o << "  const u32 smem0_ = gx_saddr(gx_smem);\n";
   // bulk copies land on 16-byte boundaries of the dynamic shared memory
-  o << "  if ((smem0_ & 15u) != 0u) { if (threadIdx.x == 0) atomicExch(a.err, 3); return; }\n";
+  o << "  if ((smem0_ & 15u) != 0u) { if (threadIdx.x == 0) gx_set_err(a.err, 3); return; }\n";
   o << "  if (threadIdx.x == 0) {\n";
   o << "    for (int q = 0; q < GX_NS; q++) { gx_mbar_init(&s_full_[q], 1u); gx_mbar_init(&s_empty_[q], GX_WARPS); }\n";
   o << "    for (int q = 0; q < GX_RR; q++) { gx_mbar_init(&s_counted_[q], 1u); gx_mbar_init(&s_based_[q], 1u); }\n";
@@ -1774,7 +1774,7 @@ void emit_fused_tma(std::ostringstream& o, const Gen& g, const Plan& p, const Ti
   o << "      for (int j = 0; ; j++) {\n";
   o << "        const int q = j % GX_NS;\n";
   o << "        if (j >= GX_NS && !gx_mbar_wait(&s_empty_[q], (u32)(j / GX_NS - 1) & 1u, GX_WAIT)) {\n";
-  o << "          atomicExch(a.err, 2);\n";
+  o << "          gx_set_err(a.err, 2);\n";
   o << "          break;\n";
   o << "        }\n";
   o << "        long long t = (long long)atomicAdd(a.tile_counter, 1ull);\n";
@@ -1793,7 +1793,7 @@ void emit_fused_tma(std::ostringstream& o, const Gen& g, const Plan& p, const Ti
   o << "    for (int j = 0; ; j++) {\n";
   o << "      const int b = j % GX_RR;\n";
   o << "      if (!gx_mbar_wait(&s_counted_[b], (u32)(j / GX_RR) & 1u, GX_WAIT)) {\n";
-  o << "        if (lane == 0) atomicExch(a.err, 2);\n";
+  o << "        if (lane == 0) gx_set_err(a.err, 2);\n";
   o << "        return;\n";
   o << "      }\n";
   o << "      const long long t = s_rtile_[b]; const u64 agg = s_ragg_[b];\n";
@@ -1864,7 +1864,7 @@ void emit_fused_tma(std::ostringstream& o, const Gen& g, const Plan& p, const Ti
   o << "    if (lane == 0) s_cnt_[vp][warp] = wcnt;\n";
   o << "    if (!gx_bar_and(ok_, GX_WARPS * 32)) {\n";
   // a copy never landed: wait (bounded) for the copies in flight, then leave
-  o << "      if (warp == 0 && lane == 0) atomicExch(a.err, 2);\n";
+  o << "      if (warp == 0 && lane == 0) gx_set_err(a.err, 2);\n";
   o << "      for (int d_ = 0; d_ < GX_NS; d_++) gx_mbar_wait(&s_full_[(j + d_) % GX_NS], (u32)((j + d_) / GX_NS) & 1u, "
        "GX_WAIT);\n";
   o << "      return;\n";
@@ -1902,7 +1902,7 @@ void emit_fused_tma(std::ostringstream& o, const Gen& g, const Plan& p, const Ti
   o << "      const int pr = jw % GX_RR;\n";
   o << "      if (s_rtile_[pr] < 0) continue;\n";
   o << "      const bool okb = gx_mbar_wait(&s_based_[pr], (u32)(jw / GX_RR) & 1u, GX_WAIT);\n";
-  o << "      if (!okb && warp == 0 && lane == 0) atomicExch(a.err, 2);\n";
+  o << "      if (!okb && warp == 0 && lane == 0) gx_set_err(a.err, 2);\n";
   o << "      const u64 base_w = okb ? s_base_[pr] : ~0ull;\n";
   o << "      if (base_w != ~0ull) {\n";
   o << "        const u32 K_w = (u32)s_ragg_[pr]; const u32 osw = GX_OBASE + (u32)(jw % GX_NR) * GX_OSTAGE;\n";
@@ -2209,7 +2209,7 @@ void emit_staged_filter(std::ostringstream& o, const Gen& g, const Plan& p, cons
   o << "          const u32 par_ = s_par[s];\n";
   o << "          u32 sp_ = 0u;\n";
   o << "          while (!gx_mbar_try_wait(&s_bar[s], par_)) {\n";
-  o << "            if (++sp_ > mbar_limit) { atomicExch(a.err, 1); s_abort = 1; break; }\n";
+  o << "            if (++sp_ > mbar_limit) { gx_set_err(a.err, 1); s_abort = 1; break; }\n";
   o << "            __nanosleep(20);\n";
   o << "          }\n";
   o << "        }\n";
@@ -2290,7 +2290,7 @@ void emit_staged_filter(std::ostringstream& o, const Gen& g, const Plan& p, cons
   o << "              s_base = ex_;\n";
   o << "              if (tile == ntiles - 1) *a.out_count = ex_ + s_total[s];\n";
   o << "            } else if (++s_lbpolls > spin_limit) {\n";
-  o << "              atomicExch(a.err, 1); s_abort = 1;\n";
+  o << "              gx_set_err(a.err, 1); s_abort = 1;\n";
   o << "            } else {\n";
   o << "              __nanosleep(64);\n";
   o << "            }\n";
