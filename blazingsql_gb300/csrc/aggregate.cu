@@ -32,6 +32,7 @@ struct AggTable {
   int* overflow;
   int* err;
   unsigned long long* groups;
+  uint32_t* list;
 };
 
 constexpr int kMaxKeys = 8;
@@ -48,7 +49,7 @@ struct AggFinal {
   void* out_data[kMaxKeys + kMaxAggs];
   uint32_t* out_mask[kMaxKeys + kMaxAggs];
   AggTable t;
-  unsigned long long* counter;
+  unsigned long long groups;
   int empty_group;  // no group keys and no row: one row of empty aggregates
   unsigned long long cnt_rows;  // accumulators whose valid count is the group's row count (input never NULL)
 };
@@ -113,21 +114,9 @@ __global__ void k_agg_finalize(AggFinal f) {
     if (blockIdx.x == 0 && threadIdx.x == 0) write_row(f, -1, 0);
     return;
   }
-  for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < f.t.cap;
-       i += (uint64_t)gridDim.x * blockDim.x) {
-    if (f.t.state[i] != 2u) continue;
-    const uint64_t p = atomicAdd(f.counter, 1ull);
-    write_row(f, (long long)i, p);
-  }
-}
-
-// MIN / MAX accumulators start at the far end of the ordered range
-__global__ void k_agg_init(AggTable t, int na, unsigned long long min_mask, unsigned long long max_mask) {
-  for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < t.cap; i += (uint64_t)gridDim.x * blockDim.x)
-    for (int j = 0; j < na; j++) {
-      if ((min_mask >> j) & 1ull) t.acc[j * t.cap + i] = 0x7FFFFFFFFFFFFFFFull;
-      if ((max_mask >> j) & 1ull) t.acc[j * t.cap + i] = 0x8000000000000000ull;
-    }
+  for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < f.groups;
+       i += (uint64_t)gridDim.x * blockDim.x)
+    write_row(f, (long long)f.t.list[i], i);
 }
 
 bool key_type_ok(int t) {
@@ -207,17 +196,10 @@ AggPlan::AggPlan(const std::vector<int>& schema, const std::vector<bool>& nullab
       out_types_.push_back(vt);
     }
   }
-  // shared-memory table: as many slots (a power of two, at most 256) as fit in
-  // about 8 KB.  A larger table costs blocks per SM, and the kernel is
-  // instruction bound.  Measured on GB300 at 2^26 order-line rows: the Q1 shape
-  // (6 groups) takes 2.48 / 2.49 / 3.01 ms with 8 / 20 / 40 KB tables; grouped
-  // by ship date (2557 groups, mostly in the global table) 8.1 / 8.8 / 16.8 ms.
-  const size_t per_slot = 4 + 4 + 8 + 8 * std::max<size_t>(key_cols.size(), 1) +
-                          16 * std::max<size_t>(layout_.kinds.size(), 1);
-  int slots = 256;
-  const int budget = std::getenv("GX_AGG_SMEM_KB") ? std::atoi(std::getenv("GX_AGG_SMEM_KB")) : 8;
-  while (slots > 16 && (size_t)slots * per_slot > (size_t)budget * 1024) slots >>= 1;
-  layout_.smem_slots = slots;
+  // one block per SM takes nearly all of its shared memory (227 KB less the
+  // kept-row lists and a margin)
+  const int budget = std::getenv("GX_AGG_SMEM_KB") ? std::atoi(std::getenv("GX_AGG_SMEM_KB")) : 208;
+  layout_.smem_bytes = std::max(8, std::min(budget, 208)) * 1024;
   const char* wc = std::getenv("GX_AGG_COMBINE");
   layout_.warp_combine = !(wc && *wc == '0');
 }
@@ -238,7 +220,10 @@ JitKernel AggPlan::kernel(const std::vector<bool>& nullable) const {
     auto it = kcache_.find(key);
     if (it != kcache_.end()) return it->second;
   }
-  const JitKernel k = jit_get(kernel_source(nullable), "gx_filter_aggregate", cfg_.warps * 32);
+  Plan p = plan_;
+  p.nullable = nullable;
+  const unsigned dyn = (unsigned)agg_shared(p, layout_, cfg_).dyn_bytes;
+  const JitKernel k = jit_get(kernel_source(nullable), "gx_filter_aggregate", cfg_.warps * 32, dyn);
   std::lock_guard<std::mutex> g(mu_);
   kcache_[key] = k;
   return k;
@@ -255,17 +240,12 @@ void AggPlan::execute(const std::vector<ColumnView>& cols, gx_column* out, int64
   std::vector<bool> nb(cols.size());
   for (size_t i = 0; i < cols.size(); i++) nb[i] = cols[i].mask != nullptr;
   const JitKernel k = kernel(nb);  // compiled before any allocation of this call
-  unsigned long long min_mask = 0, max_mask = 0;
-  for (int j = 0; j < na; j++) {
-    if (layout_.kinds[j] == 2) min_mask |= 1ull << j;
-    if (layout_.kinds[j] == 3) max_mask |= 1ull << j;
-  }
   // the global table: a start size that fits few groups cheaply, grown (and
   // the pass repeated) when a probe walks the whole table
   uint64_t cap = next_pow2((uint64_t)std::max<int64_t>(1024, std::min<int64_t>(2 * n, int64_t(1) << 17)));
   const uint64_t max_cap = next_pow2((uint64_t)std::max<int64_t>(1024, 2 * n + 16));
-  const int64_t tile_rows = (int64_t)cfg_.warps * cfg_.words * 32;
-  const int64_t ntiles = (n + tile_rows - 1) / tile_rows;
+  const int64_t chunk_rows = (int64_t)cfg_.words * 32;  // a warp's ticket
+  const int64_t nchunks = (n + chunk_rows - 1) / chunk_rows;
   unsigned long long* hflags = nullptr;  // overflow, err, groups (pinned per thread)
   thread_local unsigned long long* tflags = nullptr;
   if (!tflags) check_cuda(cudaMallocHost((void**)&tflags, 64), "pinned flags");
@@ -274,28 +254,23 @@ void AggPlan::execute(const std::vector<ColumnView>& cols, gx_column* out, int64
   char* base = nullptr;
   unsigned long long groups = 0;
   while (true) {
-    const size_t tb = (size_t)cap * (4 + 4 + 8 + 8 * nk + 16 * na);
-    const size_t bytes = tb + 256;
-    base = (char*)dev_alloc(bytes, s);
-    char* q = base;
+    // [flags | states] start at zero; a slot's other words are set when it is claimed
+    base = (char*)dev_alloc(256 + (size_t)cap * (4 + 4 + 4 + 8 + 8 * nk + 16 * na), s);
+    unsigned long long* flags = (unsigned long long*)base;  // [0] overflow, [1] err, [2] groups, [3] chunks
+    char* q = base + 256;
     t.state = (uint32_t*)q; q += cap * 4;
     t.nullm = (uint32_t*)q; q += cap * 4;
+    t.list = (uint32_t*)q; q += cap * 4;
     t.rows = (uint64_t*)q; q += cap * 8;
     t.keys = (uint64_t*)q; q += cap * 8 * nk;
     t.acc = (uint64_t*)q; q += cap * 8 * na;
     t.cnt = (uint64_t*)q; q += cap * 8 * na;
-    unsigned long long* flags = (unsigned long long*)(base + tb);  // [0] overflow, [1] err, [2] groups, [3] tiles, [4] rows out
     t.cap = cap;
     t.overflow = (int*)(flags + 0);
     t.err = (int*)(flags + 1);
     t.groups = flags + 2;
     try {
-      check_cuda(cudaMemsetAsync(base, 0, bytes, s), "aggregation table clear");
-      if (min_mask | max_mask) {
-        k_agg_init<<<(unsigned)std::min<uint64_t>((cap + 255) / 256, 4096), 256, 0, s>>>(t, na, min_mask, max_mask);
-        check_cuda(cudaGetLastError(), "k_agg_init");
-        add_launches(1);
-      }
+      check_cuda(cudaMemsetAsync(base, 0, 256 + (size_t)cap * 4, s), "aggregation table clear");
       if (n > 0) {
         KernelArgs a{};
         for (size_t i = 0; i < cols.size(); i++) bind_column(a, i, cols[i]);
@@ -305,7 +280,7 @@ void AggPlan::execute(const std::vector<ColumnView>& cols, gx_column* out, int64
         a.seed = plan_.rand_seed;
         for (int i = 0; i < 16; i++) a.order[i] = i;
         int64_t grid = (int64_t)device_sm_count() * k.max_blocks_per_sm;
-        grid = std::min<int64_t>(grid, std::max<int64_t>(ntiles, 1));
+        grid = std::min<int64_t>(grid, nchunks);
         void* params[] = {&a, &t};
         launch_raw(k, (int)grid, s, params, true);
       }
@@ -349,14 +324,14 @@ void AggPlan::execute(const std::vector<ColumnView>& cols, gx_column* out, int64
       f.out_mask[j] = out[j].null_mask;
     }
     f.t = t;
-    f.counter = (unsigned long long*)(base + (size_t)cap * (4 + 4 + 8 + 8 * nk + 16 * na)) + 4;
+    f.groups = groups;
     f.empty_group = empty_group ? 1 : 0;
     {
       Plan p = plan_;
       p.nullable = nb;
       f.cnt_rows = agg_counts_are_rows(p, layout_);
     }
-    const unsigned grid = (unsigned)std::min<uint64_t>((cap + 255) / 256, (uint64_t)device_sm_count() * 8);
+    const unsigned grid = (unsigned)std::min<uint64_t>((uint64_t)G / 256 + 1, (uint64_t)device_sm_count() * 8);
     k_agg_finalize<<<grid, 256, 0, s>>>(f);
     check_cuda(cudaGetLastError(), "k_agg_finalize");
     add_launches(1);

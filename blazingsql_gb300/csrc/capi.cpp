@@ -593,12 +593,13 @@ static std::shared_ptr<AggPlan> agg_plan_for(const std::vector<int>& schema, con
   }
   KernelConfig cfg = default_config();
   if (cfg.tune_shape) {
-    // one-warp blocks of 8 words: each warp owns its block's group table, so
-    // its shared-memory atomics meet no other warp's.  Measured on the Q1
-    // shape (2^27 rows): 1 x 8 3.88 ms; 1 x 16 4.00; 2 x 8 4.02; 2 x 4 4.04;
-    // 4 x 8 4.07; 4 x 4 4.10; 8 x 4 4.20; 8 x 2 4.45.
-    cfg.warps = 1;
-    cfg.words = 8;
+    // one block of 32 warps per SM shares its shared memory's tables; a warp's
+    // ticket is 128 rows.  Kernel us, nine aggregations by two flags (2^26 rows) /
+    // four by ship date (2^24): 32 x 4 1298 / 545, 32 x 8 1297 / 553, 28 x 4
+    // 1378 / 645; with combining trees for both, 24 x 8 1782 / 700, 16 x 8 2257 /
+    // 934.
+    cfg.warps = 32;
+    cfg.words = 4;
   }
   std::string key;
   for (size_t i = 0; i < schema.size(); i++) key += std::to_string(schema[i]) + (nullable[i] ? "n," : "-,");

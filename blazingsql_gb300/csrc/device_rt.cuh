@@ -643,7 +643,20 @@ struct GxAggArgs {
   int* overflow;               // set when a probe walked the whole table
   int* err;                    // set when a wait on a claimed slot gave up
   unsigned long long* groups;  // slots claimed
+  u32* list;                   // [cap]: the claimed slots
 };
+
+__device__ __forceinline__ u32 gx_lds_acquire(const u32* p) {
+  u32 v;
+  asm volatile("ld.acquire.cta.shared::cta.u32 %0, [%1];" : "=r"(v) : "r"(gx_saddr(p)) : "memory");
+  return v;
+}
+// 64-bit add in shared memory as two 32-bit atomics, the carry with the second
+__device__ __forceinline__ void gx_sadd64(u64* p, u64 x) {
+  const u32 lo = (u32)x, old = atomicAdd((u32*)p, lo);
+  const u32 hi = (u32)(x >> 32) + (old + lo < old ? 1u : 0u);
+  if (hi != 0u) atomicAdd((u32*)p + 1, hi);
+}
 
 __device__ __forceinline__ u64 gx_mix64(u64 x) {
   // splitmix64 finaliser

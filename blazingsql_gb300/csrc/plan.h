@@ -111,18 +111,31 @@ Plan build_plan(const std::vector<int>& schema, const std::vector<bool>& nullabl
 
 // Fused filter + group-by aggregation (gx_filter_aggregate): the plan's
 // outputs are the key columns then the non-empty aggregation inputs, all NODE
-// outputs.  The kernel keeps a hash table of groups per block in shared memory
-// and merges it into a global table (GxAggArgs) when the block finishes.
+// outputs.  The kernel keeps a block's groups in shared memory and merges them
+// into a global table (GxAggArgs) when the block finishes.
 struct AggLayout {
   std::vector<int> key_nodes;   // node of each key column
   std::vector<int> kinds;       // gx_agg_kind per aggregation
   std::vector<int> in_nodes;    // input node per aggregation (-1: COUNT(*))
-  int smem_slots = 256;         // shared-memory table slots per block (power of two)
+  int smem_bytes = 0;           // dynamic shared memory a block may take
   // the lanes of one group combine their inputs over a warp tree before one
   // lane applies them (true), or every lane applies its own row (false)
   bool warp_combine = true;
 };
 std::string generate_agg_kernel(const Plan& plan, const AggLayout& L, const KernelConfig& cfg, const std::string& name);
+// The aggregation kernel's dynamic shared memory: a dictionary of the groups
+// that have accumulators per warp, then those (`cells` 8-byte cells per group,
+// replica and warp) or, once more groups turn up, a hash table of `slots` groups.  Cell /
+// slot indices per accumulator; -1: it has none (a count has no sum, an input
+// that is never NULL no valid count).
+constexpr int kAggDict = 64;
+struct AggShared {
+  int warp_groups = 0, replicas = 1, cells = 0, rows_cell = 0;
+  int slots = 0, accs = 0;
+  int dict_bytes = 0, dyn_bytes = 0;
+  std::vector<int> acc_cell, cnt_cell, acc_slot, cnt_slot;
+};
+AggShared agg_shared(const Plan& plan, const AggLayout& L, const KernelConfig& cfg);
 // Accumulators (bit j of L's accumulator j) whose input is never NULL under
 // plan.nullable: the aggregation kernel keeps no valid count for them, and
 // the group's row count stands for it.
