@@ -445,21 +445,31 @@ static void evaluate_with_strings(std::vector<ColumnView> cols, std::string cond
       }
     }
     const int32_t* map = row_index ? (const int32_t*)tmp.back().data : nullptr;
+    // the string outputs, sized together and written after one wait
+    StringBuilds sb(s);
+    std::vector<size_t> building;
+    auto finish = [&] {
+      const std::vector<gx_column> made = sb.finish();
+      for (size_t b = 0; b < made.size(); b++) out[building[b]] = made[b];
+      building.clear();
+    };
     for (size_t i = 0; i < ex.size(); i++) {
       if (src[i] == -2) continue;
+      if (sb.size() == StringBuilds::kMax) finish();
       StrSource a, none;
       if (src[i] == -1) {
         a.kind = StrSource::LITERAL;
         a.literal = lit[i];
-        out[i] = build_strings(a, none, nullptr, nullptr, rows, s);
+        sb.strings(a, none, nullptr, nullptr, rows);
+        building.push_back(i);
         continue;
       }
       const size_t k = (size_t)src[i] - ncols0;
       if (src[i] >= (int)ncols0 && k < pp.defer.size() && pp.defer[k]) {  // made now, for the kept rows
-        out[i] = transform_column(pp.ops[k], cols, filtering ? map : nullptr, rows, s,
-                                  [s](const std::vector<ColumnView>& c, const std::string& t) {
-                                    return eval_condition(c, t, s);
-                                  });
+        begin_transform(sb, pp.ops[k], cols, filtering ? map : nullptr, rows, s,
+                        [s](const std::vector<ColumnView>& c, const std::string& t) { return eval_condition(c, t, s); },
+                        &tmp);
+        building.push_back(i);
         continue;
       }
       if (!filtering && src[i] >= (int)ncols0 && k < pp.made.size() && pp.made[k].data) {
@@ -469,8 +479,10 @@ static void evaluate_with_strings(std::vector<ColumnView> cols, std::string cond
       }
       a.kind = StrSource::COLUMN;
       a.col = cols[src[i]];
-      out[i] = build_strings(a, none, filtering ? map : nullptr, nullptr, rows, s);
+      sb.strings(a, none, filtering ? map : nullptr, nullptr, rows);
+      building.push_back(i);
     }
+    finish();
   } catch (...) {
     for (size_t i = 0; i < ex.size(); i++)
       if (out[i].data || out[i].null_mask) free_column(out[i], s);

@@ -24,6 +24,8 @@
 #include <array>
 #include <cstring>
 #include <map>
+#include <mutex>
+#include <type_traits>
 
 namespace gx {
 
@@ -241,11 +243,23 @@ __global__ void k_string_op(StrArgs a) {
 }
 
 // ------------------------------------------------------------ string builder
-// A strings column is built in three launches: row sizes and validity (and a
-// character total per block), an exclusive scan of the block totals, then
-// offsets and characters.  A block covers kBuildWarps x kBuildWords 32-row
-// words.  A warp's rows are copied together by warp_copy when they are long,
-// a lane per row when they are short.
+// A strings column is built in three launches: row sizes and validity, the
+// characters before each 32-row word within its block and the block's total; an
+// exclusive scan of the block totals; then offsets and characters, every word on
+// its own.  A block covers kBuildWarps x kBuildWords words.  A warp's rows are
+// copied together by warp_copy when they are long, through a shared-memory
+// stage when they are short.
+//
+// The launches wait on chains of dependent loads (row map, offsets, characters),
+// so the chains are kept short: the writing launch takes a row's length and its
+// word's start from the sizing one, and a row's bytes come as up to five aligned
+// words at once (stage_bytes) -- copied a byte at a time, each load waited for
+// the store before it, which may alias it.  2^23 rows, us (sizes + write): a
+// gather of 5-character rows 39 + 101 before, 23 + 81 now; SUBSTRING(1, 10) 102 +
+// 183, now 70 + 116 (its characters come in one coalesced pass, span_ascii); CONCAT
+// of three parts 77 + 184, now 65 + 178.  What bounds them: the instructions of
+// the byte stores and the waits for scattered characters (a row's load touches
+// a line of its own), not memory bandwidth.
 constexpr int kBuildWarps = 8, kBuildWords = 8;
 constexpr int64_t kBuildRows = kBuildWarps * kBuildWords * 32;
 
@@ -273,6 +287,7 @@ struct BuildArgs {
   uint32_t* out_mask;
   unsigned char* out_chars;
   uint64_t* block_sums;
+  uint32_t* word_base;  // characters before each word within its block
 };
 
 __device__ __forceinline__ bool bit_of(const uint32_t* mask, int64_t q) {
@@ -303,12 +318,6 @@ __device__ __forceinline__ void resolve(const BuildArgs& a, int64_t o, const uns
   p = s.chars + b0;
   len = s.offs[q + 1] - b0;
   valid = true;
-}
-
-__device__ __forceinline__ int warp_sum(int v) {
-#pragma unroll
-  for (int d = 16; d > 0; d >>= 1) v += __shfl_xor_sync(0xffffffffu, v, d);
-  return v;
 }
 
 // Rows longer than this on average (bytes) are copied by warp_copy; shorter
@@ -360,64 +369,130 @@ __device__ __forceinline__ void stage_flush(unsigned char* out, uint64_t pos, co
   if (lane < wtot - t0) out[pos + t0 + lane] = st[sh + t0 + lane];
 }
 
-__global__ void __launch_bounds__(kBuildWarps * 32) k_str_sizes(BuildArgs a) {
-  __shared__ uint64_t s_sum[kBuildWarps];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int64_t w0 = ((int64_t)blockIdx.x * kBuildWarps + warp) * kBuildWords;
-  uint64_t total = 0;
-  for (int k = 0; k < kBuildWords; k++) {
-    const int64_t o = (w0 + k) * 32 + lane;
-    if ((w0 + k) * 32 >= a.m) break;
-    const unsigned char* p;
-    int len = 0;
-    bool valid = false;
-    if (o < a.m) resolve(a, o, p, len, valid);
-    const uint32_t word = __ballot_sync(0xffffffffu, valid);
-    if (lane == 0) a.out_mask[w0 + k] = word;
-    total += (uint64_t)warp_sum(len);
+// n bytes at p (device memory) to st (shared memory), 16 at a time: the aligned
+// words that hold them are loaded together, then stored byte by byte.  Every
+// word loaded holds at least one of the bytes.
+__device__ __forceinline__ void stage_bytes(unsigned char* st, const unsigned char* p, int n) {
+  for (int done = 0; done < n; done += 16, p += 16, st += 16) {
+    const int k = min(n - done, 16);
+    const uint32_t* w = (const uint32_t*)((uintptr_t)p & ~(uintptr_t)3);
+    const int sh = ((int)(uintptr_t)p & 3) * 8, words = (((int)(uintptr_t)p & 3) + k + 3) >> 2;
+    uint32_t r[5];
+#pragma unroll
+    for (int i = 0; i < 5; i++) r[i] = i < words ? __ldg(w + i) : 0u;
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+      if (i * 4 >= k) break;
+      const uint32_t v = __funnelshift_r(r[i], r[i + 1], sh);
+#pragma unroll
+      for (int j = 0; j < 4; j++)
+        if (i * 4 + j < k) st[i * 4 + j] = (unsigned char)(v >> (8 * j));
+    }
   }
-  if (lane == 0) s_sum[warp] = total;
+}
+
+// The characters of a word's 32 rows: exact also where they pass 32 bits, so
+// that a column over 2^31 - 1 characters is seen and refused.
+__device__ __forceinline__ uint64_t word_total(int len) {
+  if (!__any_sync(0xffffffffu, len >> 26)) return __reduce_add_sync(0xffffffffu, (uint32_t)len);
+  uint64_t v = (uint64_t)len;
+#pragma unroll 1
+  for (int d = 16; d > 0; d >>= 1) v += __shfl_xor_sync(0xffffffffu, v, d);
+  return v;
+}
+
+// The words' character totals of a block (s_w, one per word in word order)
+// become their starts within the block; the block's total goes to block_sums.
+// Called by every thread, after the totals were written.
+__device__ __forceinline__ void scan_words(const uint64_t* s_w, uint32_t* word_base, int64_t words, uint64_t* block_sums) {
+  static_assert(kBuildWarps * kBuildWords == 64, "two words per lane");
   __syncthreads();
-  if (threadIdx.x == 0) {
-    uint64_t t = 0;
-    for (int i = 0; i < kBuildWarps; i++) t += s_sum[i];
-    a.block_sums[blockIdx.x] = t;
+  if (threadIdx.x >= 32) return;
+  const int lane = threadIdx.x;
+  const uint64_t x = s_w[2 * lane], y = s_w[2 * lane + 1];
+  uint64_t incl = x + y;
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    const uint64_t t = __shfl_up_sync(0xffffffffu, incl, d);
+    if (lane >= d) incl += t;
   }
+  const int64_t w = (int64_t)blockIdx.x * 64 + 2 * lane;
+  if (w < words) word_base[w] = (uint32_t)(incl - x - y);
+  if (w + 1 < words) word_base[w + 1] = (uint32_t)(incl - y);
+  if (lane == 31) block_sums[blockIdx.x] = incl;
+}
+
+// inclusive sum over the warp's lanes
+__device__ __forceinline__ int warp_incl(int v, int lane) {
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    const int y = __shfl_up_sync(0xffffffffu, v, d);
+    if (lane >= d) v += y;
+  }
+  return v;
+}
+
+__global__ void __launch_bounds__(kBuildWarps * 32) k_str_sizes(BuildArgs a) {
+  __shared__ uint64_t s_w[kBuildWarps * kBuildWords];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int64_t words = (a.m + 31) / 32, first = (int64_t)blockIdx.x * (kBuildWarps * kBuildWords) + warp;
+  int len[kBuildWords];
+  bool valid[kBuildWords];
+  if (a.a.kind == StrSource::COLUMN && !a.cond) {
+    // one column: the loads of all the warp's words go out together
+    int64_t q[kBuildWords];
+#pragma unroll
+    for (int k = 0; k < kBuildWords; k++) {
+      const int64_t o = min((first + k * kBuildWarps) * 32 + lane, a.m - 1);
+      q[k] = a.a.off + (a.map ? (int64_t)__ldg(a.map + o) : o);
+    }
+#pragma unroll
+    for (int k = 0; k < kBuildWords; k++) {
+      len[k] = __ldg(a.a.offs + q[k] + 1) - __ldg(a.a.offs + q[k]);
+      valid[k] = !a.a.mask || ((__ldg(a.a.mask + (q[k] >> 5)) >> (q[k] & 31)) & 1u);
+    }
+#pragma unroll
+    for (int k = 0; k < kBuildWords; k++) {
+      valid[k] = valid[k] && (first + k * kBuildWarps) * 32 + lane < a.m;
+      if (!valid[k]) len[k] = 0;
+    }
+  } else {
+#pragma unroll
+    for (int k = 0; k < kBuildWords; k++) {
+      const int64_t o = (first + k * kBuildWarps) * 32 + lane;
+      const unsigned char* p;
+      len[k] = 0;
+      valid[k] = false;
+      if (o < a.m) resolve(a, o, p, len[k], valid[k]);
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < kBuildWords; k++) {
+    const int64_t w = first + k * kBuildWarps;
+    const uint32_t word = __ballot_sync(0xffffffffu, valid[k]);
+    const uint64_t total = word_total(len[k]);
+    if (lane == 0) {
+      if (w < words) a.out_mask[w] = word;
+      s_w[k * kBuildWarps + warp] = total;
+    }
+  }
+  scan_words(s_w, a.word_base, words, a.block_sums);
 }
 
 // block_sums hold each block's first character position (exclusive scan)
 __global__ void __launch_bounds__(kBuildWarps * 32) k_str_write(BuildArgs a) {
-  __shared__ uint64_t s_sum[kBuildWarps];
   __shared__ __align__(16) unsigned char s_stage[kBuildWarps][kStageBytes + 8];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int64_t w0 = ((int64_t)blockIdx.x * kBuildWarps + warp) * kBuildWords;
-  uint64_t total = 0;
+  const uint64_t block_pos = a.block_sums[blockIdx.x];
   for (int k = 0; k < kBuildWords; k++) {
-    const int64_t o = (w0 + k) * 32 + lane;
-    if ((w0 + k) * 32 >= a.m) break;
-    const unsigned char* p;
-    int len = 0;
-    bool valid = false;
-    if (o < a.m) resolve(a, o, p, len, valid);
-    total += (uint64_t)warp_sum(len);
-  }
-  if (lane == 0) s_sum[warp] = total;
-  __syncthreads();
-  uint64_t pos = a.block_sums[blockIdx.x];
-  for (int i = 0; i < warp; i++) pos += s_sum[i];
-  for (int k = 0; k < kBuildWords; k++) {
-    const int64_t o = (w0 + k) * 32 + lane;
-    if ((w0 + k) * 32 >= a.m) break;
+    const int64_t w = (int64_t)blockIdx.x * (kBuildWarps * kBuildWords) + k * kBuildWarps + warp, o = w * 32 + lane;
+    if (w * 32 >= a.m) break;
+    const uint64_t pos = block_pos + a.word_base[w];
     const unsigned char* p = nullptr;
     int len = 0;
     bool valid = false;
     if (o < a.m) resolve(a, o, p, len, valid);
-    int incl = len;
-#pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-      const int y = __shfl_up_sync(0xffffffffu, incl, d);
-      if (lane >= d) incl += y;
-    }
+    const int incl = warp_incl(len, lane);
     const uint64_t dst = pos + (uint64_t)(incl - len);
     if (o < a.m) {
       a.out_offs[o] = (int32_t)dst;
@@ -427,13 +502,11 @@ __global__ void __launch_bounds__(kBuildWarps * 32) k_str_write(BuildArgs a) {
     if (wtot > kStageBytes) {  // long rows: the warp copies them together
       warp_copy(a.out_chars + pos, incl - len, len, p, nullptr, wtot, lane);
     } else {  // short rows: each lane stages its own, the warp writes them out
-      unsigned char* st = s_stage[warp] + (pos & 3u) + (incl - len);
-      for (int i = 0; i < len; i++) st[i] = p[i];
+      stage_bytes(s_stage[warp] + (pos & 3u) + (incl - len), p, len);
       __syncwarp();
       stage_flush(a.out_chars, pos, s_stage[warp], wtot, lane);
       __syncwarp();
     }
-    pos += (uint64_t)wtot;
   }
 }
 
@@ -469,7 +542,14 @@ struct XformArgs {
   uint32_t* out_mask;
   unsigned char* out_chars;
   uint64_t* block_sums;
+  uint32_t* word_base;
 };
+
+// The transforms' kernels are instantiated for the common kinds, so that these
+// do not carry the registers of every other one: a slice by literal positions
+// from the front, a CONCAT, REGEXP_REPLACE (whose Pike VM keeps its thread lists
+// in local memory), and one for all the rest.
+enum XformClass { XF_ANY = 0, XF_REGEX = 1, XF_FRONT_SLICE = 2, XF_CONCAT = 3 };
 
 __device__ __forceinline__ void source_row(const BuildSrc& s, int64_t o, const unsigned char*& p, int& len,
                                            bool& valid) {
@@ -513,9 +593,22 @@ __device__ bool in_set(const unsigned char* s, int i, int k, const unsigned char
 }
 
 // the decimal digits of v (as unsigned), zero-padded to `width`, at d + at;
-// counted first, then written from the last digit (no buffer)
+// counted first, then written from the last digit (no buffer); 32-bit divisions
+// where the value allows
 __device__ __forceinline__ int civil_digits(unsigned char* d, int at, int64_t v, int width) {
   uint64_t u = (uint64_t)v;
+  if (u <= 0xFFFFFFFFull) {
+    uint32_t x = (uint32_t)u;
+    int n = 1;
+    for (uint32_t t = x; t >= 10; t /= 10) n++;
+    if (n < width) n = width;
+    if (d)
+      for (int i = n - 1; i >= 0; i--) {
+        d[at + i] = (unsigned char)('0' + x % 10);
+        x /= 10;
+      }
+    return at + n;
+  }
   int n = 1;
   for (uint64_t t = u; t >= 10; t /= 10) n++;
   if (n < width) n = width;
@@ -722,6 +815,34 @@ __device__ __forceinline__ bool ascii_prefix(const unsigned char* p, int lim) {
   return (acc & 0x80808080u) == 0;
 }
 
+// [i0, i1) characters from the front of the n bytes at p (SUBSTRING with a
+// length, LEFT), as n1 bytes at p1.  When the first min(n, i1) bytes are ASCII,
+// characters are bytes: the slice is [i0, min(n, i1)), found without a
+// dependent walk
+__device__ __forceinline__ void front_slice(const XformArgs& a, const unsigned char* p, int n, const unsigned char*& p1,
+                                            int& n1) {
+  n1 = 0;
+  const int lim = min(n, a.i1);
+  if (ascii_prefix(p, lim)) {
+    if (a.i0 >= lim) return;
+    p1 = p + a.i0;
+    n1 = lim - a.i0;
+    return;
+  }
+  // otherwise walk at most i1 characters, without counting the rest
+  int i = 0, c = 0, bb = 0;
+  while (i < n && c < a.i1) {
+    if (c == a.i0) bb = i;
+    i += utf8_len(p[i]);
+    c++;
+  }
+  if (a.i0 >= c) return;  // begins at or after the end
+  i = min(i, n);
+  p1 = p + bb;
+  n1 = i - bb;
+}
+
+template <int kClass>
 __device__ int xform_segments(const XformArgs& a, int64_t o, const unsigned char*& p1, int& n1,
                               const unsigned char*& p2, bool& valid) {
   const unsigned char* p;
@@ -729,7 +850,7 @@ __device__ int xform_segments(const XformArgs& a, int64_t o, const unsigned char
   source_row(a.a, o, p, n, valid);
   p1 = p2 = nullptr;
   n1 = 0;
-  if (a.kind == StringOp::CONCAT) {  // cudf::strings::concatenate: NULL if either side is
+  if (kClass == XF_CONCAT || (kClass == XF_ANY && a.kind == StringOp::CONCAT)) {  // cudf::strings::concatenate: NULL if either side is
     const unsigned char* q;
     int m;
     bool v2;
@@ -742,7 +863,7 @@ __device__ int xform_segments(const XformArgs& a, int64_t o, const unsigned char
     return n + m;
   }
   if (!valid) return 0;
-  if (a.kind == StringOp::SLICE && a.p0) {
+  if (kClass == XF_ANY && a.kind == StringOp::SLICE && a.p0) {
     // cudf::strings::slice_strings with a start and a stop per row: the start
     // clamped at 0, a stop below 0 or past the end meaning the end, empty when
     // the start is not before the stop
@@ -762,29 +883,8 @@ __device__ int xform_segments(const XformArgs& a, int64_t o, const unsigned char
     n1 = eb - bb;
     return n1;
   }
-  if (a.kind == StringOp::SLICE && a.i0v && a.i1v && a.i0 >= 0 && a.i1 >= 0) {
-    // [i0, i1) from the front (SUBSTRING with a length, LEFT).  When the
-    // first min(n, i1) bytes are ASCII, characters are bytes: the slice is
-    // [i0, min(n, i1)), found without a dependent walk
-    const int lim = min(n, a.i1);
-    if (ascii_prefix(p, lim)) {
-      if (a.i0 >= lim) return 0;
-      p1 = p + a.i0;
-      n1 = lim - a.i0;
-      return n1;
-    }
-    // otherwise walk at most i1 characters; the same clipping as below,
-    // without counting the rest
-    int i = 0, c = 0, bb = 0;
-    while (i < n && c < a.i1) {
-      if (c == a.i0) bb = i;
-      i += utf8_len(p[i]);
-      c++;
-    }
-    if (a.i0 >= c) return 0;  // begins at or after the end
-    i = min(i, n);
-    p1 = p + bb;
-    n1 = i - bb;
+  if (kClass == XF_FRONT_SLICE || (a.kind == StringOp::SLICE && a.i0v && a.i1v && a.i0 >= 0 && a.i1 >= 0)) {
+    front_slice(a, p, n, p1, n1);
     return n1;
   }
   if (a.kind == StringOp::SLICE) {  // cudf::strings::slice_strings, characters [begin, end)
@@ -892,19 +992,20 @@ __device__ __forceinline__ int put_utf8(unsigned char* d, int at, uint32_t c) {
   return at + n;
 }
 
+template <int kClass>
 __device__ int xform_row(const XformArgs& a, int64_t o, unsigned char* d, bool& valid) {
-  if (a.kind == StringOp::TO_STRING) return format_value(a, o, d, valid);
-  if (is_segment_kind(a)) {
+  if (kClass == XF_ANY && a.kind == StringOp::TO_STRING) return format_value(a, o, d, valid);
+  if (kClass == XF_FRONT_SLICE || is_segment_kind(a)) {
     const unsigned char *p1, *p2;
     int n1;
-    const int len = xform_segments(a, o, p1, n1, p2, valid);
+    const int len = xform_segments<kClass>(a, o, p1, n1, p2, valid);
     if (d) {
       put(d, 0, p1, n1);
       put(d, n1, p2, len - n1);
     }
     return len;
   }
-  if (a.kind == StringOp::CONCAT) {  // more than two parts or a formatted part, NULL if any is
+  if (kClass == XF_CONCAT || a.kind == StringOp::CONCAT) {  // more than two parts or a formatted part, NULL if any is
     int at = 0;
 #pragma unroll
     for (int k = 0; k < kMaxConcatParts; k++) {  // unrolled: the parts stay in parameter space
@@ -919,7 +1020,8 @@ __device__ int xform_row(const XformArgs& a, int64_t o, unsigned char* d, bool& 
       int m;
       source_row(ps, o, q, m, valid);
       if (!valid) return 0;
-      at = put(d, at, q, m);
+      if (d) stage_bytes(d + at, q, m);
+      at += m;
     }
     return at;
   }
@@ -1008,93 +1110,190 @@ __device__ int xform_row(const XformArgs& a, int64_t o, unsigned char* d, bool& 
   }
 }
 
-// kRegex: REGEXP_REPLACE rows (a separate instantiation keeps the Pike VM's
-// thread lists out of the other transforms' local memory)
-template <bool kRegex>
-__global__ void __launch_bounds__(kBuildWarps * 32) k_xf_sizes(XformArgs a) {
-  __shared__ uint64_t s_sum[kBuildWarps];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int64_t w0 = ((int64_t)blockIdx.x * kBuildWarps + warp) * kBuildWords;
-  uint64_t total = 0;
-  for (int k = 0; k < kBuildWords; k++) {
-    const int64_t o = (w0 + k) * 32 + lane;
-    if ((w0 + k) * 32 >= a.m) break;
-    const int64_t src = (o < a.m && a.map) ? (int64_t)a.map[o] : o;  // the input row
-    bool valid = false;
-    int len = 0;
-    if (o < a.m) {
-      if constexpr (kRegex) len = regex_row(a, src, nullptr, valid);
-      else len = xform_row(a, src, nullptr, valid);
-      a.out_offs[o] = len;  // the row's length, read back by k_xf_write (which then writes offsets)
-    }
-    const uint32_t word = __ballot_sync(0xffffffffu, valid);
-    if (lane == 0) a.out_mask[w0 + k] = word;
-    total += (uint64_t)warp_sum(len);
+// The characters [lo, hi) of a column, at most kSpanBytes of them, as aligned
+// 16-byte blocks (every block loaded holds at least one of them): true when all
+// of the blocks are ASCII, false also when there are more characters.  With buf
+// (kSpanBytes of the warp's shared memory) the blocks are left there.  Called by
+// the whole warp.
+constexpr int kSpanBytes = 2048;
+__device__ __forceinline__ bool span_ascii(const unsigned char* chars, int32_t lo, int32_t hi, int lane,
+                                           unsigned char* buf = nullptr) {
+  const uintptr_t first = (uintptr_t)(chars + lo) & ~(uintptr_t)15;
+  const int64_t bytes = (int64_t)((uintptr_t)(chars + hi) - first);
+  if (hi <= lo || bytes > kSpanBytes) return false;
+  uint32_t acc = 0;
+  for (int i = lane * 16; i < (int)bytes; i += 512) {
+    const uint4 v = __ldg((const uint4*)(first + i));
+    if (buf) *(uint4*)(buf + i) = v;
+    acc |= v.x | v.y | v.z | v.w;
   }
-  if (lane == 0) s_sum[warp] = total;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    uint64_t t = 0;
-    for (int i = 0; i < kBuildWarps; i++) t += s_sum[i];
-    a.block_sums[blockIdx.x] = t;
+  return !__any_sync(0xffffffffu, (acc & 0x80808080u) != 0);
+}
+
+// Rows o[0..U) of a source (already row numbers of the input) for a lane: the
+// length each contributes, NULL rows clearing ok; U loads in flight at a time.
+template <int U>
+__device__ __forceinline__ void part_lengths(const BuildSrc& ps, const int64_t* row, int* len, bool* ok) {
+  if (ps.kind == StrSource::LITERAL) {
+#pragma unroll
+    for (int j = 0; j < U; j++) len[j] += ps.lit_len;
+  } else if (ps.kind == StrSource::COLUMN) {
+#pragma unroll
+    for (int j = 0; j < U; j++) {
+      const int64_t q = ps.off + row[j];
+      len[j] += __ldg(ps.offs + q + 1) - __ldg(ps.offs + q);
+      ok[j] = ok[j] && (!ps.mask || ((__ldg(ps.mask + (q >> 5)) >> (q & 31)) & 1u));
+    }
+  } else if (ps.kind == StrSource::FORMAT) {
+#pragma unroll
+    for (int j = 0; j < U; j++) {
+      bool v;
+      len[j] += format_typed(ps.num, ps.mask, ps.off, ps.num_type, row[j], nullptr, v);
+      ok[j] = ok[j] && v;
+    }
+  } else {
+#pragma unroll
+    for (int j = 0; j < U; j++) ok[j] = false;
   }
 }
 
-template <bool kRegex>
-__global__ void __launch_bounds__(kBuildWarps * 32) k_xf_write(XformArgs a) {
-  __shared__ uint64_t s_sum[kBuildWarps];
-  __shared__ __align__(16) unsigned char s_stage[kBuildWarps][kStageBytes + 8];
+template <int kClass>
+__global__ void __launch_bounds__(kBuildWarps * 32) k_xf_sizes(XformArgs a) {
+  __shared__ uint64_t s_w[kBuildWarps * kBuildWords];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int64_t w0 = ((int64_t)blockIdx.x * kBuildWarps + warp) * kBuildWords;
-  uint64_t total = 0;
-  for (int k = 0; k < kBuildWords; k++) {
-    const int64_t o = (w0 + k) * 32 + lane;
-    if ((w0 + k) * 32 >= a.m) break;
-    const int len = o < a.m ? a.out_offs[o] : 0;  // k_xf_sizes' row lengths
-    total += (uint64_t)warp_sum(len);
-  }
-  if (lane == 0) s_sum[warp] = total;
-  __syncthreads();
-  uint64_t pos = a.block_sums[blockIdx.x];
-  for (int i = 0; i < warp; i++) pos += s_sum[i];
-  for (int k = 0; k < kBuildWords; k++) {
-    const int64_t o = (w0 + k) * 32 + lane;
-    if ((w0 + k) * 32 >= a.m) break;
-    const int64_t src = (o < a.m && a.map) ? (int64_t)a.map[o] : o;  // the input row
-    const bool seg = !kRegex && is_segment_kind(a);  // warp-uniform
-    const unsigned char *p1 = nullptr, *p2 = nullptr;
-    int n1 = 0, len = 0;
-    bool valid = false;
-    if (o < a.m) {
-      if (seg) len = xform_segments(a, src, p1, n1, p2, valid);
-      else len = a.out_offs[o];  // k_xf_sizes' row length
-    }
-    int incl = len;
+  const int64_t words = (a.m + 31) / 32, first = (int64_t)blockIdx.x * (kBuildWarps * kBuildWords) + warp;
+  constexpr int U = kClass == XF_CONCAT || kClass == XF_FRONT_SLICE ? 4 : 1;
+  for (int k = 0; k < kBuildWords; k += U) {
+    int64_t row[U];  // the input rows
+    int len[U];
+    bool valid[U];
 #pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-      const int y = __shfl_up_sync(0xffffffffu, incl, d);
-      if (lane >= d) incl += y;
+    for (int j = 0; j < U; j++) {
+      const int64_t o = min((first + (k + j) * kBuildWarps) * 32 + lane, a.m - 1);
+      row[j] = a.map ? (int64_t)__ldg(a.map + o) : o;
+      len[j] = 0;
+      valid[j] = true;
     }
+    if constexpr (kClass == XF_CONCAT) {
+      part_lengths<U>(a.a, row, len, valid);
+      part_lengths<U>(a.b, row, len, valid);
+#pragma unroll
+      for (int p = 0; p < kMaxConcatParts - 2; p++)
+        if (p < a.nmore) part_lengths<U>(a.more[p], row, len, valid);
+    } else if constexpr (kClass == XF_FRONT_SLICE) {
+      int32_t b[U], n[U];
+#pragma unroll
+      for (int j = 0; j < U; j++) {
+        const int64_t q = a.a.off + row[j];
+        b[j] = __ldg(a.a.offs + q);
+        n[j] = __ldg(a.a.offs + q + 1) - b[j];
+        valid[j] = !a.a.mask || ((__ldg(a.a.mask + (q >> 5)) >> (q & 31)) & 1u);
+      }
+#pragma unroll
+      for (int j = 0; j < U; j++) {
+        // where the first i1 bytes of the word's rows (and what lies between
+        // them) are ASCII, characters are bytes and no row is looked at
+        const int32_t lim = min(n[j], a.i1);
+        const int32_t lo = __reduce_min_sync(0xffffffffu, b[j]), hi = __reduce_max_sync(0xffffffffu, b[j] + lim);
+        if (span_ascii(a.a.chars, lo, hi, lane)) {
+          len[j] = max(0, lim - a.i0);
+        } else if (valid[j]) {
+          const unsigned char* p1 = nullptr;
+          front_slice(a, a.a.chars + b[j], n[j], p1, len[j]);
+        }
+      }
+    } else {
+      const int64_t o = (first + k * kBuildWarps) * 32 + lane;
+      if (o < a.m) {
+        if constexpr (kClass == XF_REGEX) len[0] = regex_row(a, row[0], nullptr, valid[0]);
+        else len[0] = xform_row<kClass>(a, row[0], nullptr, valid[0]);
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < U; j++) {
+      const int64_t w = first + (k + j) * kBuildWarps, o = w * 32 + lane;
+      const bool v = valid[j] && o < a.m;
+      const int l = v ? len[j] : 0;
+      if (o < a.m) a.out_offs[o] = l;  // the row's length, read back by k_xf_write (which then writes offsets)
+      const uint32_t word = __ballot_sync(0xffffffffu, v);
+      const uint64_t total = word_total(l);
+      if (lane == 0) {
+        if (w < words) a.out_mask[w] = word;
+        s_w[(k + j) * kBuildWarps + warp] = total;
+      }
+    }
+  }
+  scan_words(s_w, a.word_base, words, a.block_sums);
+}
+
+template <int kClass>
+__global__ void __launch_bounds__(kBuildWarps * 32) k_xf_write(XformArgs a) {
+  __shared__ __align__(16) unsigned char s_stage[kBuildWarps][kStageBytes + 8];
+  constexpr bool kSpan = kClass == XF_FRONT_SLICE;
+  __shared__ __align__(16) unsigned char s_span[kSpan ? kBuildWarps : 1][kSpan ? kSpanBytes : 16];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const bool seg = kClass == XF_FRONT_SLICE || (kClass != XF_REGEX && is_segment_kind(a));  // warp-uniform
+  const uint64_t block_pos = a.block_sums[blockIdx.x];
+  for (int k = 0; k < kBuildWords; k++) {
+    const int64_t w = (int64_t)blockIdx.x * (kBuildWarps * kBuildWords) + k * kBuildWarps + warp, o = w * 32 + lane;
+    if (w * 32 >= a.m) break;
+    const uint64_t pos = block_pos + a.word_base[w];
+    const int64_t src = (o < a.m && a.map) ? (int64_t)a.map[o] : o;  // the input row
+    const unsigned char *p1 = nullptr, *p2 = nullptr;
+    int n1 = 0;
+    bool valid = false, spanned = false;
+    const int len = o < a.m ? a.out_offs[o] : 0;  // k_xf_sizes' row length
+    if constexpr (kClass == XF_FRONT_SLICE) {
+      const int64_t q = a.a.off + (o < a.m ? src : (int64_t)0);
+      const int32_t b = __ldg(a.a.offs + q), n = __ldg(a.a.offs + q + 1) - b;
+      const int32_t lo = __reduce_min_sync(0xffffffffu, len > 0 ? b : INT32_MAX);
+      const int32_t hi = __reduce_max_sync(0xffffffffu, len > 0 ? b + min(n, a.i1) : 0);
+      spanned = span_ascii(a.a.chars, lo, hi, lane, s_span[warp]);
+      if (spanned) {
+        p1 = s_span[warp] + (((uintptr_t)(a.a.chars + lo) & 15u) + (uint32_t)(b - lo) + (uint32_t)a.i0);
+        n1 = len;
+      } else if (len > 0) {
+        front_slice(a, a.a.chars + b, n, p1, n1);
+      }
+    } else {
+      if (seg && len > 0) xform_segments<kClass>(a, src, p1, n1, p2, valid);
+    }
+    const int incl = warp_incl(len, lane);
     const uint64_t dst = pos + (uint64_t)(incl - len);
+    __syncwarp();  // every lane has read its length
     if (o < a.m) {
       a.out_offs[o] = (int32_t)dst;
       if (o == a.m - 1) a.out_offs[a.m] = (int32_t)(dst + (uint64_t)len);
     }
     const int wtot = __shfl_sync(0xffffffffu, incl, 31);
-    if (seg && wtot > 32 * kWarpCopyBytes) {  // long rows: the warp copies them together
-      warp_copy(a.out_chars + pos, incl - len, n1, p1, p2, wtot, lane);
-    } else if (seg) {  // short rows: staged by their lanes, written out by the warp
+    if (wtot <= kStageBytes) {  // short rows: staged by their lanes, written out by the warp
       unsigned char* st = s_stage[warp] + (pos & 3u) + (incl - len);
-      for (int i = 0; i < n1; i++) st[i] = p1[i];
-      for (int i = n1; i < len; i++) st[i] = p2[i - n1];
+      if (spanned) {
+        int i = 0;
+        for (; i + 4 <= len; i += 4) {
+          const unsigned char c0 = p1[i], c1 = p1[i + 1], c2 = p1[i + 2], c3 = p1[i + 3];
+          st[i] = c0;
+          st[i + 1] = c1;
+          st[i + 2] = c2;
+          st[i + 3] = c3;
+        }
+        for (; i < len; i++) st[i] = p1[i];
+      } else if (seg) {
+        stage_bytes(st, p1, n1);
+        stage_bytes(st + n1, p2, len - n1);
+      } else if (len > 0) {
+        if constexpr (kClass == XF_REGEX) regex_row(a, src, st, valid);
+        else xform_row<kClass>(a, src, st, valid);
+      }
       __syncwarp();
       stage_flush(a.out_chars, pos, s_stage[warp], wtot, lane);
       __syncwarp();
-    } else if (o < a.m && len > 0) {
-      if constexpr (kRegex) regex_row(a, src, a.out_chars + dst, valid);
-      else xform_row(a, src, a.out_chars + dst, valid);
+    } else if (seg) {  // long rows: the warp copies them together
+      warp_copy(a.out_chars + pos, incl - len, n1, p1, p2, wtot, lane);
+    } else if (len > 0) {
+      if constexpr (kClass == XF_REGEX) regex_row(a, src, a.out_chars + dst, valid);
+      else xform_row<kClass>(a, src, a.out_chars + dst, valid);
     }
-    pos += (uint64_t)wtot;
   }
 }
 
@@ -1281,177 +1480,235 @@ BuildSrc device_source(const StrSource& s, const unsigned char* lit_dev) {
 
 }  // namespace
 
-gx_column build_strings(const StrSource& a, const StrSource& b, const int32_t* map, const ColumnView* cond,
-                        int64_t rows, cudaStream_t s) {
+namespace {
+// A string column between its sizing and its writing launches.
+struct Build {
+  gx_column out{};
+  bool xform = false;
+  XformClass cls = XF_ANY;
+  BuildArgs b{};
+  XformArgs x{};
+  unsigned nblocks = 0;
+  const volatile unsigned long long* total = nullptr;  // the character total, once the sizes are scanned
+};
+}  // namespace
+
+// Mapped words for the character totals of one StringBuilds, kept for the next
+// one of any thread (pinning memory costs more than a build); more than
+// kKeptSlots at a time are given back.
+static std::mutex g_slots_mu;
+static std::vector<unsigned long long*> g_slots;
+constexpr size_t kKeptSlots = 16;
+
+struct StringBuilds::State {
+  std::vector<Build> builds;
+  unsigned long long* totals = nullptr;
+
+  unsigned long long* slot(int i) {
+    if (!totals) {
+      std::lock_guard<std::mutex> lk(g_slots_mu);
+      if (!g_slots.empty()) {
+        totals = g_slots.back();
+        g_slots.pop_back();
+      }
+    }
+    if (!totals)
+      check_cuda(cudaHostAlloc((void**)&totals, kMax * 8, cudaHostAllocMapped | cudaHostAllocPortable), "string totals");
+    return totals + i;
+  }
+};
+
+StringBuilds::StringBuilds(cudaStream_t s) : s_(s), st_(new State) {}
+StringBuilds::~StringBuilds() {
+  if (!st_->builds.empty()) {  // begun and not finished
+    cudaStreamSynchronize(s_);  // their sizing may still write the totals
+    for (auto& b : st_->builds) {
+      if (b.out.data) dev_free(b.out.data, s_);
+      dev_free(b.out.null_mask, s_);
+    }
+  }
+  if (!st_->totals) return;
+  {
+    std::lock_guard<std::mutex> lk(g_slots_mu);
+    if (g_slots.size() < kKeptSlots) {
+      g_slots.push_back(st_->totals);
+      return;
+    }
+  }
+  cudaFreeHost(st_->totals);
+}
+int StringBuilds::size() const { return (int)st_->builds.size(); }
+
+// Allocates [mask | offsets | word starts | block sums | literals], uploads the
+// literals, and clears what the sizing launch does not write (the mask's
+// padding, the first offset of an empty column).
+static char* begin_build(Build& b, int64_t rows, const std::vector<std::string>& lits, std::vector<unsigned char*>* lit_dev,
+                         uint32_t** word_base, uint64_t** sums, cudaStream_t s) {
   if (rows < 0 || rows > INT32_MAX) fail(GX_ERR_UNSUPPORTED, "string columns hold at most 2^31 - 1 rows");
+  const int64_t words = mask_words_for(rows), used = (rows + 31) / 32;
+  b.nblocks = (unsigned)((rows + kBuildRows - 1) / kBuildRows);
+  auto al = [](size_t v) { return (v + 255) / 256 * 256; };
+  const size_t mask_b = al((size_t)words * 4), offs_b = al((size_t)(rows + 1) * 4), word_b = al((size_t)(used + 1) * 4);
+  const size_t sums_b = al((size_t)(b.nblocks + 1) * 8);
+  size_t lit_b = 0;
+  for (const auto& l : lits) lit_b += al(l.size() + 1);
+  char* base = (char*)dev_alloc(mask_b + offs_b + word_b + sums_b + lit_b, s);
+  b.out.type_id = STRING;
+  b.out.null_mask = (uint32_t*)base;
+  b.out.string_offsets = (int32_t*)(base + mask_b);
+  b.out.size = rows;
+  b.out.capacity = rows;
+  *word_base = (uint32_t*)(base + mask_b + offs_b);
+  *sums = (uint64_t*)(base + mask_b + offs_b + word_b);
+  unsigned char* l = (unsigned char*)(base + mask_b + offs_b + word_b + sums_b);
+  if (words > used) check_cuda(cudaMemsetAsync(base + used * 4, 0, (size_t)(words - used) * 4, s), "mask padding");
+  if (rows == 0) check_cuda(cudaMemsetAsync(b.out.string_offsets, 0, 4, s), "empty offsets");
+  for (const auto& x : lits) {
+    lit_dev->push_back(l);
+    // (a copy from pageable memory returns once its bytes are staged)
+    if (!x.empty()) check_cuda(cudaMemcpyAsync(l, x.data(), x.size(), cudaMemcpyHostToDevice, s), "string literal");
+    l += al(x.size() + 1);
+  }
+  return base;
+}
+
+template <class F>
+static void with_class(XformClass c, F&& f) {
+  switch (c) {
+    case XF_REGEX: f(std::integral_constant<int, XF_REGEX>{}); break;
+    case XF_FRONT_SLICE: f(std::integral_constant<int, XF_FRONT_SLICE>{}); break;
+    case XF_CONCAT: f(std::integral_constant<int, XF_CONCAT>{}); break;
+    default: f(std::integral_constant<int, XF_ANY>{}); break;
+  }
+}
+
+// the sizing launch and the scan of the block totals
+static void launch_sizes(Build& b, uint64_t* sums, unsigned long long* total, int64_t rows, cudaStream_t s) {
+  *total = 0;
+  b.total = total;
+  if (rows == 0) return;
+  if (b.xform) with_class(b.cls, [&](auto c) { k_xf_sizes<decltype(c)::value><<<b.nblocks, kBuildWarps * 32, 0, s>>>(b.x); });
+  else k_str_sizes<<<b.nblocks, kBuildWarps * 32, 0, s>>>(b.b);
+  check_cuda(cudaGetLastError(), "string sizes");
+  launch_scan_tiles(sums, b.nblocks, total, s);
+  add_launches(1);
+}
+
+void StringBuilds::strings(const StrSource& a, const StrSource& b, const int32_t* map, const ColumnView* cond, int64_t rows) {
   if (map && a.kind != StrSource::COLUMN) fail(GX_ERR_INVALID, "a gather reads a column");
   if (cond && cond->type != BOOL8)
     fail(GX_ERR_TYPE, "Expression does not evaluate to a boolean mask");  // LogicalProject.cpp:636
-  const int64_t nblocks = (rows + kBuildRows - 1) / kBuildRows;
-  const int64_t words = mask_words_for(rows);
-  auto al = [](size_t v) { return (v + 255) / 256 * 256; };
-  // [mask | offsets | block sums + total | literals]
-  const size_t mask_b = al((size_t)words * 4), offs_b = al((size_t)(rows + 1) * 4);
-  const size_t sums_b = al((size_t)(nblocks + 1) * 8);
-  const size_t la = a.kind == StrSource::LITERAL ? al(a.literal.size() + 1) : 0;
-  const size_t lb = b.kind == StrSource::LITERAL ? al(b.literal.size() + 1) : 0;
-  char* base = (char*)dev_alloc(mask_b + offs_b + sums_b + la + lb, s);
-  gx_column out{};
-  out.type_id = STRING;
-  out.null_mask = (uint32_t*)base;
-  out.string_offsets = (int32_t*)(base + mask_b);
-  out.size = rows;
-  out.capacity = rows;
-  try {
-    uint64_t* sums = (uint64_t*)(base + mask_b + offs_b);
-    unsigned char* lit_a = (unsigned char*)(base + mask_b + offs_b + sums_b);
-    unsigned char* lit_b = lit_a + la;
-    check_cuda(cudaMemsetAsync(base, 0, mask_b + offs_b, s), "string column clear");
-    if (la && !a.literal.empty())
-      check_cuda(cudaMemcpyAsync(lit_a, a.literal.data(), a.literal.size(), cudaMemcpyHostToDevice, s), "literal");
-    if (lb && !b.literal.empty())
-      check_cuda(cudaMemcpyAsync(lit_b, b.literal.data(), b.literal.size(), cudaMemcpyHostToDevice, s), "literal");
-    BuildArgs args{};
-    args.a = device_source(a, lit_a);
-    args.b = device_source(b, lit_b);
-    args.map = map;
-    if (cond) {
-      args.cond = (const unsigned char*)cond->data;
-      args.cond_mask = cond->mask;
-      args.cond_off = cond->offset;
-    }
-    args.m = rows;
-    args.out_offs = out.string_offsets;
-    args.out_mask = out.null_mask;
-    args.block_sums = sums;
-    uint64_t total = 0;
-    if (rows > 0) {
-      k_str_sizes<<<(unsigned)nblocks, kBuildWarps * 32, 0, s>>>(args);
-      check_cuda(cudaGetLastError(), "k_str_sizes");
-      launch_scan_tiles(sums, nblocks, (unsigned long long*)(sums + nblocks), s);
-      check_cuda(cudaMemcpyAsync(&total, sums + nblocks, 8, cudaMemcpyDeviceToHost, s), "string size");
-      add_launches(1);
-    }
-    // the literals' host bytes and `total` must outlive the copies
-    check_cuda(cudaStreamSynchronize(s), "string size sync");
-    if (total > (uint64_t)INT32_MAX) fail(GX_ERR_UNSUPPORTED, "string column over 2^31 - 1 characters");
-    out.data = dev_alloc(al(total ? total : 1), s);
-    out.string_bytes = (int64_t)total;
-    if (rows > 0) {
-      args.out_chars = (unsigned char*)out.data;
-      k_str_write<<<(unsigned)nblocks, kBuildWarps * 32, 0, s>>>(args);
-      check_cuda(cudaGetLastError(), "k_str_write");
-      add_launches(1);
-    }
-  } catch (...) {
-    if (out.data) dev_free(out.data, s);
-    dev_free(base, s);
-    throw;
+  if (size() >= kMax) fail(GX_ERR_INVALID, "too many string builds at once");
+  st_->builds.emplace_back();
+  Build& x = st_->builds.back();
+  std::vector<unsigned char*> lit;
+  uint64_t* sums = nullptr;
+  begin_build(x, rows, {a.kind == StrSource::LITERAL ? a.literal : std::string(),
+                        b.kind == StrSource::LITERAL ? b.literal : std::string()},
+              &lit, &x.b.word_base, &sums, s_);
+  x.b.a = device_source(a, lit[0]);
+  x.b.b = device_source(b, lit[1]);
+  x.b.map = map;
+  if (cond) {
+    x.b.cond = (const unsigned char*)cond->data;
+    x.b.cond_mask = cond->mask;
+    x.b.cond_off = cond->offset;
   }
-  return out;
+  x.b.m = rows;
+  x.b.out_offs = x.out.string_offsets;
+  x.b.out_mask = x.out.null_mask;
+  x.b.block_sums = sums;
+  launch_sizes(x, sums, st_->slot(size() - 1), rows, s_);
 }
 
-gx_column build_transform(const StringOp& op, const StrSource& a, const StrSource& b, const ColumnView* num,
-                          int64_t rows, cudaStream_t s, const std::vector<StrSource>& more,
-                          const ColumnView* pos0 = nullptr, const ColumnView* pos1 = nullptr,
-                          const int32_t* map = nullptr) {
+void StringBuilds::transform(const StringOp& op, const StrSource& a, const StrSource& b, const ColumnView* num,
+                             int64_t rows, const std::vector<StrSource>& more, const ColumnView* pos0,
+                             const ColumnView* pos1, const int32_t* map) {
   if (more.size() > (size_t)(kMaxConcatParts - 2)) fail(GX_ERR_INVALID, "too many CONCAT parts");
-  if (rows < 0 || rows > INT32_MAX) fail(GX_ERR_UNSUPPORTED, "string columns hold at most 2^31 - 1 rows");
-  const int64_t nblocks = (rows + kBuildRows - 1) / kBuildRows;
-  const int64_t words = mask_words_for(rows);
-  auto al = [](size_t v) { return (v + 255) / 256 * 256; };
-  // [mask | offsets | block sums + total | a, b, literal, literal2]
-  const size_t mask_b = al((size_t)words * 4), offs_b = al((size_t)(rows + 1) * 4);
-  const size_t sums_b = al((size_t)(nblocks + 1) * 8);
+  if (size() >= kMax) fail(GX_ERR_INVALID, "too many string builds at once");
+  st_->builds.emplace_back();
+  Build& bd = st_->builds.back();
+  bd.xform = true;
   std::vector<std::string> lits = {a.kind == StrSource::LITERAL ? a.literal : std::string(),
                                    b.kind == StrSource::LITERAL ? b.literal : std::string(), op.literal,
                                    op.literal2};
   for (const auto& x : more) lits.push_back(x.kind == StrSource::LITERAL ? x.literal : std::string());
-  const int nl = (int)lits.size();
-  std::vector<size_t> loff(nl);
-  size_t lb = 0;
-  for (int i = 0; i < nl; i++) {
-    loff[i] = lb;
-    lb += al(lits[i].size() + 1);
+  std::vector<unsigned char*> lit;
+  uint64_t* sums = nullptr;
+  XformArgs& x = bd.x;
+  begin_build(bd, rows, lits, &lit, &x.word_base, &sums, s_);
+  x.kind = op.kind;
+  x.a = device_source(a, lit[0]);
+  x.b = device_source(b, lit[1]);
+  x.nmore = (int)more.size();
+  for (size_t k = 0; k < more.size(); k++) x.more[k] = device_source(more[k], lit[4 + k]);
+  if (num) {
+    x.num = num->data;
+    x.num_mask = num->mask;
+    x.num_off = num->offset;
+    x.num_type = num->type;
   }
-  char* base = (char*)dev_alloc(mask_b + offs_b + sums_b + lb, s);
-  gx_column out{};
-  out.type_id = STRING;
-  out.null_mask = (uint32_t*)base;
-  out.string_offsets = (int32_t*)(base + mask_b);
-  out.size = rows;
-  out.capacity = rows;
-  try {
-    uint64_t* sums = (uint64_t*)(base + mask_b + offs_b);
-    unsigned char* ldev = (unsigned char*)(base + mask_b + offs_b + sums_b);
-    check_cuda(cudaMemsetAsync(base, 0, mask_b + offs_b + sums_b, s), "string column clear");
-    for (int i = 0; i < nl; i++)
-      if (!lits[i].empty())
-        check_cuda(cudaMemcpyAsync(ldev + loff[i], lits[i].data(), lits[i].size(), cudaMemcpyHostToDevice, s),
-                   "string literal");
-    XformArgs x{};
-    x.kind = op.kind;
-    x.a = device_source(a, ldev + loff[0]);
-    x.b = device_source(b, ldev + loff[1]);
-    x.nmore = (int)more.size();
-    for (size_t k = 0; k < more.size(); k++) x.more[k] = device_source(more[k], ldev + loff[4 + k]);
-    if (num) {
-      x.num = num->data;
-      x.num_mask = num->mask;
-      x.num_off = num->offset;
-      x.num_type = num->type;
-    }
-    if (pos0) {
-      x.p0 = pos0->data;
-      x.p0m = pos0->mask;
-      x.p0t = pos0->type;
-    }
-    if (pos1) {
-      x.p1 = pos1->data;
-      x.p1m = pos1->mask;
-      x.p1t = pos1->type;
-    }
-    x.i0 = op.i0;
-    x.i1 = op.i1;
-    x.step = op.step;
-    x.i0v = op.i0_valid;
-    x.i1v = op.i1_valid;
-    x.s1 = ldev + loff[2];
-    x.l1 = (int)op.literal.size();
-    x.s2 = ldev + loff[3];
-    x.l2 = (int)op.literal2.size();
-    x.m = rows;
-    x.map = map;
-    x.out_offs = out.string_offsets;
-    x.out_mask = out.null_mask;
-    x.block_sums = sums;
-    uint64_t host[1] = {0};
-    if (rows > 0) {
-      if (op.kind == StringOp::REGEXP_REPLACE) k_xf_sizes<true><<<(unsigned)nblocks, kBuildWarps * 32, 0, s>>>(x);
-      else k_xf_sizes<false><<<(unsigned)nblocks, kBuildWarps * 32, 0, s>>>(x);
-      check_cuda(cudaGetLastError(), "k_xf_sizes");
-      launch_scan_tiles(sums, nblocks, (unsigned long long*)(sums + nblocks), s);
-      check_cuda(cudaMemcpyAsync(host, sums + nblocks, 8, cudaMemcpyDeviceToHost, s), "string size");
-      add_launches(1);
-    }
-    check_cuda(cudaStreamSynchronize(s), "string size sync");
-    const uint64_t total = host[0];
+  if (pos0) {
+    x.p0 = pos0->data;
+    x.p0m = pos0->mask;
+    x.p0t = pos0->type;
+  }
+  if (pos1) {
+    x.p1 = pos1->data;
+    x.p1m = pos1->mask;
+    x.p1t = pos1->type;
+  }
+  x.i0 = op.i0;
+  x.i1 = op.i1;
+  x.step = op.step;
+  x.i0v = op.i0_valid;
+  x.i1v = op.i1_valid;
+  x.s1 = lit[2];
+  x.l1 = (int)op.literal.size();
+  x.s2 = lit[3];
+  x.l2 = (int)op.literal2.size();
+  x.m = rows;
+  x.map = map;
+  x.out_offs = bd.out.string_offsets;
+  x.out_mask = bd.out.null_mask;
+  x.block_sums = sums;
+  bd.cls = op.kind == StringOp::REGEXP_REPLACE ? XF_REGEX
+           : op.kind == StringOp::CONCAT ? XF_CONCAT
+           : op.kind == StringOp::SLICE && !pos0 && op.step > 0 && op.i0_valid && op.i1_valid && op.i0 >= 0 && op.i1 >= 0
+               ? XF_FRONT_SLICE : XF_ANY;
+  launch_sizes(bd, sums, st_->slot(size() - 1), rows, s_);
+}
+
+std::vector<gx_column> StringBuilds::finish() {
+  std::vector<gx_column> out;
+  if (st_->builds.empty()) return out;
+  check_cuda(cudaStreamSynchronize(s_), "string size sync");
+  for (auto& b : st_->builds) {
+    const uint64_t total = *b.total;
     if (total > (uint64_t)INT32_MAX) fail(GX_ERR_UNSUPPORTED, "string column over 2^31 - 1 characters");
-    out.data = dev_alloc(al(total ? total : 1), s);
-    out.string_bytes = (int64_t)total;
-    if (rows > 0) {
-      x.out_chars = (unsigned char*)out.data;
-      if (op.kind == StringOp::REGEXP_REPLACE) k_xf_write<true><<<(unsigned)nblocks, kBuildWarps * 32, 0, s>>>(x);
-      else k_xf_write<false><<<(unsigned)nblocks, kBuildWarps * 32, 0, s>>>(x);
-      check_cuda(cudaGetLastError(), "k_xf_write");
-      add_launches(1);
+    b.out.data = dev_alloc(std::max<size_t>((size_t)(total + 255) / 256 * 256, 256), s_);
+    b.out.string_bytes = (int64_t)total;
+    if (b.out.size == 0) continue;
+    if (b.xform) {
+      b.x.out_chars = (unsigned char*)b.out.data;
+      with_class(b.cls, [&](auto c) { k_xf_write<decltype(c)::value><<<b.nblocks, kBuildWarps * 32, 0, s_>>>(b.x); });
+    } else {
+      b.b.out_chars = (unsigned char*)b.out.data;
+      k_str_write<<<b.nblocks, kBuildWarps * 32, 0, s_>>>(b.b);
     }
-  } catch (...) {
-    if (out.data) dev_free(out.data, s);
-    dev_free(base, s);
-    throw;
+    check_cuda(cudaGetLastError(), "string write");
+    add_launches(1);
   }
+  for (auto& b : st_->builds) out.push_back(b.out);
+  st_->builds.clear();
   return out;
+}
+
+gx_column build_strings(const StrSource& a, const StrSource& b, const int32_t* map, const ColumnView* cond,
+                        int64_t rows, cudaStream_t s) {
+  StringBuilds sb(s);
+  sb.strings(a, b, map, cond, rows);
+  return sb.finish()[0];
 }
 
 void launch_parse(const ColumnView& col, int type, const std::string& format, gx_column& out, cudaStream_t s) {
@@ -1616,7 +1873,7 @@ static bool build_like_dfa(const std::string& pat, LikeDfa& d) {
 int like_dfa_host_match(const std::string& pattern, const unsigned char* text, int64_t n) {
   LikeDfa d;
   if (!build_like_dfa(pattern, d)) return -1;
-  // the same walk as k_string_op's
+  // the same walk as the kernels'
   if (d.classes == 0) {  // byte-indexed
     const unsigned char* tr = (const unsigned char*)d.blob.data();
     const unsigned char* flags = tr + (size_t)d.states * 256;
@@ -1690,33 +1947,44 @@ bool is_deferrable(const StringOp& op) {
 
 gx_column transform_column(const StringOp& op, const std::vector<ColumnView>& cols, const int32_t* map,
                            int64_t rows, cudaStream_t s, const EvalText& eval_bool) {
+  StringBuilds sb(s);
+  std::vector<gx_column> temps;
+  auto release = [&] {
+    for (auto& c : temps) free_column(c, s);
+  };
+  try {
+    begin_transform(sb, op, cols, map, rows, s, eval_bool, &temps);
+    const gx_column out = sb.finish()[0];
+    release();
+    return out;
+  } catch (...) {
+    release();
+    throw;
+  }
+}
+
+void begin_transform(StringBuilds& sb, const StringOp& op, const std::vector<ColumnView>& cols, const int32_t* map,
+                     int64_t rows, cudaStream_t s, const EvalText& eval_bool, std::vector<gx_column>* temps) {
   const int64_t n = cols.empty() ? 0 : cols[0].size;
   auto string_col = [&](int c) { return string_column(cols, c); };
-  gx_column out{};
   if (op.kind == StringOp::TO_STRING) {
-    gx_column tmp{};
     ColumnView v = op.col >= 0 ? cols.at(op.col) : ColumnView{};
     if (op.col < 0) {
-      tmp = eval_bool(cols, op.cond);
-      v = ColumnView{tmp.type_id, tmp.data, tmp.null_mask, 0, n, tmp.string_offsets};
+      temps->push_back(eval_bool(cols, op.cond));
+      const gx_column& t = temps->back();
+      v = ColumnView{t.type_id, t.data, t.null_mask, 0, n, t.string_offsets};
     }
-    try {
-      if (v.type == STRING) {
-        StrSource a, none;
-        a.kind = StrSource::COLUMN;
-        a.col = v;
-        out = build_strings(a, none, map, nullptr, rows, s);
-      } else {
-        if (type_size(v.type) == 0 || v.type >= DURATION_DAYS)
-          fail(GX_ERR_UNSUPPORTED, "CAST to VARCHAR of type " + std::to_string(v.type));
-        out = build_transform(op, StrSource{}, StrSource{}, &v, rows, s, {}, nullptr, nullptr, map);
-      }
-    } catch (...) {
-      if (tmp.data || tmp.null_mask) free_column(tmp, s);
-      throw;
+    if (v.type == STRING) {
+      StrSource a, none;
+      a.kind = StrSource::COLUMN;
+      a.col = v;
+      sb.strings(a, none, map, nullptr, rows);
+    } else {
+      if (type_size(v.type) == 0 || v.type >= DURATION_DAYS)
+        fail(GX_ERR_UNSUPPORTED, "CAST to VARCHAR of type " + std::to_string(v.type));
+      sb.transform(op, StrSource{}, StrSource{}, &v, rows, {}, nullptr, nullptr, map);
     }
-    if (tmp.data || tmp.null_mask) free_column(tmp, s);
-    return out;
+    return;
   }
   // a part: a string column, a literal, or (CONCAT) a typed column to format
   auto part = [&](int c, const std::string& lit) {
@@ -1743,32 +2011,22 @@ gx_column transform_column(const StringOp& op, const std::vector<ColumnView>& co
   if (op.kind == StringOp::SLICE && !op.pos0.empty()) {
     // the start and stop columns (LogicalProject.cpp:241-300), made by
     // the same evaluator as a CASE condition over every input row
-    gx_column pc[2] = {};
-    auto release = [&] {
-      for (auto& c : pc)
-        if (c.data || c.null_mask) free_column(c, s);
-    };
-    try {
-      ColumnView pv[2];
-      for (int k = 0; k < 2; k++) {
-        const std::string& text = k == 0 ? op.pos0 : op.pos1;
-        if (text.empty()) continue;
-        pc[k] = eval_bool(cols, text);
-        const int t = pc[k].type_id;
-        if (t != INT8 && t != INT16 && t != INT32 && t != INT64 && t != UINT8 && t != UINT16 && t != UINT32 &&
-            t != UINT64)
-          fail(GX_ERR_TYPE, "Expression does not evaluate to an integer column");  // :252
-        pv[k] = ColumnView{t, pc[k].data, pc[k].null_mask, 0, n};
-      }
-      out = build_transform(xo, a, b, nullptr, rows, s, more, &pv[0], op.pos1.empty() ? nullptr : &pv[1], map);
-    } catch (...) {
-      release();
-      throw;
+    ColumnView pv[2];
+    for (int k = 0; k < 2; k++) {
+      const std::string& text = k == 0 ? op.pos0 : op.pos1;
+      if (text.empty()) continue;
+      temps->push_back(eval_bool(cols, text));
+      const gx_column& pc = temps->back();
+      const int t = pc.type_id;
+      if (t != INT8 && t != INT16 && t != INT32 && t != INT64 && t != UINT8 && t != UINT16 && t != UINT32 &&
+          t != UINT64)
+        fail(GX_ERR_TYPE, "Expression does not evaluate to an integer column");  // :252
+      pv[k] = ColumnView{t, pc.data, pc.null_mask, 0, n};
     }
-    release();
-    return out;
+    sb.transform(xo, a, b, nullptr, rows, more, &pv[0], op.pos1.empty() ? nullptr : &pv[1], map);
+    return;
   }
-  return build_transform(xo, a, b, nullptr, rows, s, more, nullptr, nullptr, map);
+  sb.transform(xo, a, b, nullptr, rows, more, nullptr, nullptr, map);
 }
 
 std::vector<gx_column> run_string_prepass(std::vector<ColumnView>& cols, const std::vector<StringOp>& ops,
@@ -1858,8 +2116,7 @@ std::vector<gx_column> run_string_prepass(std::vector<ColumnView>& cols, const s
     dev_free(pdev, s);
     throw;
   }
-  // the copy of the patterns must finish before their host buffer goes away
-  check_cuda(cudaStreamSynchronize(s), "string pre-pass");
+  // (the patterns' copy returned once their pageable bytes were staged)
   dev_free(pdev, s);
   return made;
 }

@@ -6,6 +6,7 @@
 #include <cuda_runtime.h>
 
 #include <functional>
+#include <memory>
 #include <string>
 #include <vector>
 
@@ -50,6 +51,30 @@ struct StrSource {
 gx_column build_strings(const StrSource& a, const StrSource& b, const int32_t* map, const ColumnView* cond,
                         int64_t rows, cudaStream_t s);
 
+// Several string columns built together: each begin call enqueues a column's
+// sizing, finish() waits once for all their character totals, allocates and
+// enqueues the writing (a column at a time waits, and leaves the device idle,
+// once per column).  What the columns are made from must live until finish().
+// At most kMax columns between two finish() calls.
+class StringBuilds {
+ public:
+  static constexpr int kMax = 64;
+  explicit StringBuilds(cudaStream_t s);
+  ~StringBuilds();  // releases columns that finish() did not return
+  StringBuilds(const StringBuilds&) = delete;
+  StringBuilds& operator=(const StringBuilds&) = delete;
+  int size() const;
+  void strings(const StrSource& a, const StrSource& b, const int32_t* map, const ColumnView* cond, int64_t rows);
+  void transform(const StringOp& op, const StrSource& a, const StrSource& b, const ColumnView* num, int64_t rows,
+                 const std::vector<StrSource>& more, const ColumnView* pos0, const ColumnView* pos1, const int32_t* map);
+  std::vector<gx_column> finish();
+
+ private:
+  struct State;
+  cudaStream_t s_;
+  std::unique_ptr<State> st_;
+};
+
 // Evaluates `ops` over `cols` and appends their columns to `cols` (column
 // ncols + i is op i).  eval_bool evaluates an expression's text over the
 // columns so far into a column: a CASE condition (BOOL8), the operand of a
@@ -72,5 +97,9 @@ bool is_deferrable(const StringOp& op);
 // kept rows of a filter, LogicalFilter.cpp:22-29, gathered while building).
 gx_column transform_column(const StringOp& op, const std::vector<ColumnView>& cols, const int32_t* map,
                            int64_t rows, cudaStream_t s, const EvalText& eval_bool);
+// The same as a build of `sb`; columns evaluated for it are added to *temps, the
+// caller's to free after sb.finish().
+void begin_transform(StringBuilds& sb, const StringOp& op, const std::vector<ColumnView>& cols, const int32_t* map,
+                     int64_t rows, cudaStream_t s, const EvalText& eval_bool, std::vector<gx_column>* temps);
 
 }  // namespace gx
