@@ -2605,10 +2605,25 @@ uint64_t agg_counts_are_rows(const Plan& p, const AggLayout& L) {
   return m;
 }
 
+// Bits of group key j (an integer, date or BOOL8 column) as a field of a packed key
+static int agg_key_bits(const Plan& p, const AggLayout& L, int j) {
+  return 8 * type_size(p.schema[p.nodes[L.key_nodes[j]].col]);
+}
+// All keys, their null bits and one bit that is always set fit a 64-bit word: a
+// group then is one word in shared memory, claimed by one compare-and-swap and
+// compared by one load (else: a state word, a null word and a word per key, with
+// a wait while another lane writes them).
+static bool agg_packs_keys(const Plan& p, const AggLayout& L) {
+  int bits = 1 + (int)L.key_nodes.size();
+  for (size_t j = 0; j < L.key_nodes.size(); j++) bits += agg_key_bits(p, L, (int)j);
+  return bits <= 64;
+}
+
 AggShared agg_shared(const Plan& p, const AggLayout& L, const KernelConfig& cfg) {
   const int nk = std::max<int>(1, (int)L.key_nodes.size()), na = (int)L.kinds.size();
   const uint64_t rows_cnt = agg_counts_are_rows(p, L);
   AggShared s;
+  s.packed = agg_packs_keys(p, L);
   s.acc_cell.assign(na, -1);
   s.cnt_cell.assign(na, -1);
   s.acc_slot.assign(na, -1);
@@ -2630,7 +2645,7 @@ AggShared agg_shared(const Plan& p, const AggLayout& L, const KernelConfig& cfg)
   const int room = budget / (cfg.warps * s.cells * 8);  // words of a cell per warp
   s.replicas = std::max(1, std::min(8, room / 16));
   s.warp_groups = std::min(kAggDict / 2, room / s.replicas);
-  const int slot_bytes = 8 * (nk + s.accs) + 4 * (3 + cnts);
+  const int slot_bytes = 8 * ((s.packed ? 1 : nk) + s.accs) + 4 * ((s.packed ? 1 : 3) + cnts);
   s.slots = std::max(16, std::min(8192, budget / slot_bytes) / 8 * 8);
   s.dyn_bytes = s.dict_bytes + std::max(s.warp_groups * s.replicas * cfg.warps * s.cells * 8, s.slots * slot_bytes);
   return s;
@@ -2675,62 +2690,126 @@ std::string generate_agg_kernel(const Plan& p, const AggLayout& L, const KernelC
     for (int j = 0; j < nk; j++)
       os << ind << ks << "[" << j << "ull * " << stride << " + " << pos << "] = kv[" << j << "];\n";
   };
-  // the block's table: -1 when the probe finds no room, -2 after a wait gave up
-  o << "__device__ int gxa_find_smem(u32* st, u32* nm, u64* ks, const u64* kv, u32 kn, u64 h, int* err) {\n"
-       "  u32 pos = __umulhi((u32)h, (u32)GXA_S);\n"
-       "  for (int pr = 0; pr < GXA_PROBES; pr++) {\n"
-       "    u32 s = gx_lds_acquire(st + pos);\n"
-       "    if (s == 0u) {\n"
-       "      s = atomicCAS(st + pos, 0u, 1u);\n"
-       "      if (s == 0u) {\n";
-  write_keys(o, "ks", "GXA_S", "pos", "        ");
-  o << "        nm[pos] = kn;\n"
-       "        __threadfence_block();\n"
-       "        atomicExch(st + pos, 2u);\n"
-       "        return (int)pos;\n"
-       "      }\n"
-       "    }\n"
-       "    u32 spins = 0;\n"
-       "    while (s == 1u) {\n"
-       "      if (++spins > (1u << 20)) { atomicExch(err, 1); return -2; }\n"
-       "      __nanosleep(16);\n"
-       "      s = gx_lds_acquire(st + pos);\n"
-       "    }\n"
-       "    if (*(volatile u32*)(nm + pos) == kn && " << same_keys("ks", "GXA_S", "pos") << ") return (int)pos;\n"
-       "    pos = pos + 1u == GXA_S ? 0u : pos + 1u;\n"
-       "  }\n"
-       "  return -1;\n"
-       "}\n";
-  // the block's dictionary of groups with warp accumulators: the group's index,
-  // -1 when it has none and no room is left, -2 after a wait gave up
-  o << "__device__ int gxa_find_warp(u32* st, u32* nm, u64* ks, u32* at, u32* ng, const u64* kv, u32 kn, u64 h, int* err) {\n"
-       "  u32 pos = (u32)h & (GXA_D - 1);\n"
-       "  for (int pr = 0; pr < GXA_D; pr++) {\n"
-       "    u32 s = gx_lds_acquire(st + pos);\n"
-       "    if (s == 0u) {\n"
-       "      if (*(volatile u32*)ng >= GXA_G) return -1;\n"
-       "      s = atomicCAS(st + pos, 0u, 1u);\n"
-       "      if (s == 0u) {\n"
-       "        const u32 i = atomicAdd(ng, 1u);\n"
-       "        if (i >= GXA_G) { atomicExch(st + pos, 0xffffffffu); return -1; }\n";  // lost the last place
-  write_keys(o, "ks", "GXA_D", "pos", "        ");
-  o << "        nm[pos] = kn; at[i] = pos;\n"
-       "        __threadfence_block();\n"
-       "        atomicExch(st + pos, 2u + i);\n"
-       "        return (int)i;\n"
-       "      }\n"
-       "    }\n"
-       "    u32 spins = 0;\n"
-       "    while (s == 1u) {\n"
-       "      if (++spins > (1u << 20)) { atomicExch(err, 1); return -2; }\n"
-       "      __nanosleep(16);\n"
-       "      s = gx_lds_acquire(st + pos);\n"
-       "    }\n"
-       "    if (s != 0xffffffffu && *(volatile u32*)(nm + pos) == kn && " << same_keys("ks", "GXA_D", "pos") << ") return (int)s - 2;\n"
-       "    pos = (pos + 1u) & (GXA_D - 1);\n"
-       "  }\n"
-       "  return -1;\n"
-       "}\n";
+  if (sh.packed) {
+    // a group as one word, and back; its place in shared memory is the key times
+    // 2^32 over the golden ratio (Knuth's multiplicative hashing): consecutive
+    // keys -- dates, numbered rows -- fall evenly over the table, so the longest
+    // probe of a warp's 32 lanes, which all of them wait for, stays short
+    int off = 1 + nk;
+    std::string pack = "1ull | ((u64)kn << 1)", unpack;
+    for (int j = 0; j < nk; j++) {
+      const int w = agg_key_bits(p, L, j);
+      const std::string m = "0x" + [&] { std::ostringstream h; h << std::hex << (w == 64 ? ~0ull : (1ull << w) - 1ull); return h.str(); }() + "ull";
+      pack += " | ((kv[" + std::to_string(j) + "] & " + m + ") << " + std::to_string(off) + ")";
+      const bool sgn = std::string(load_fn(p.schema[p.nodes[L.key_nodes[j]].col])).find("_u") == std::string::npos;
+      const std::string lsh = std::to_string(64 - off - w), rsh = std::to_string(64 - w);
+      unpack += " kv[" + std::to_string(j) + "] = " + (sgn ? "(u64)((i64)(pk << " + lsh + ") >> " + rsh + ")" : "(pk << " + lsh + ") >> " + rsh) + ";";
+      off += w;
+    }
+    o << "__device__ __forceinline__ u64 gxa_pack(const u64* kv, u32 kn) { return " << pack << "; }\n";
+    o << "__device__ __forceinline__ u32 gxa_unpack(u64 pk, u64* kv) { kv[0] = 0ull;" << unpack << " return (u32)(pk >> 1) & "
+      << ((1u << nk) - 1u) << "u; }\n";
+    o << "__device__ __forceinline__ u32 gxa_place(u64 pk) {\n  u32 h = (u32)(pk >> " << 1 + nk << ") * 0x9E3779B1u;\n";
+    if (off - 1 - nk > 32) o << "  h = (h ^ (h >> 15) ^ (u32)(pk >> " << 33 + nk << ")) * 0x9E3779B1u;\n";
+    if (nk) o << "  h += ((u32)(pk >> 1) & " << ((1u << nk) - 1u) << "u) * 0x27D4EB2Fu;\n";
+    o << "  return h;\n}\n";
+    o << "__device__ int gxa_find_table(u64* pk, u64 key) {\n"
+         "  u32 pos = __umulhi(gxa_place(key), (u32)GXA_S);\n"
+         "  for (int pr = 0; pr < GXA_PROBES; pr++) {\n"
+         "    u64 v = *(volatile u64*)(pk + pos);\n"
+         "    if (v == 0ull) v = atomicCAS((unsigned long long*)(pk + pos), 0ull, (unsigned long long)key);\n"
+         "    if (v == 0ull || v == key) return (int)pos;\n"
+         "    pos = pos + 1u == GXA_S ? 0u : pos + 1u;\n"
+         "  }\n"
+         "  return -1;\n"
+         "}\n";
+    o << "__device__ int gxa_find_dict(u32* st, u64* pk, u32* at, u32* ng, u64 key, int* err) {\n"
+         "  u32 pos = __umulhi(gxa_place(key), (u32)GXA_D);\n"
+         "  for (int pr = 0; pr < GXA_D; pr++) {\n"
+         "    u64 v = *(volatile u64*)(pk + pos);\n"
+         "    if (v == 0ull) {\n"
+         "      if (*(volatile u32*)ng >= GXA_G) return -1;\n"
+         "      v = atomicCAS((unsigned long long*)(pk + pos), 0ull, (unsigned long long)key);\n"
+         "      if (v == 0ull) {\n"
+         "        const u32 i = atomicAdd(ng, 1u);\n"
+         "        if (i >= GXA_G) { atomicExch(st + pos, 0xffffffffu); return -1; }\n"  // lost the last place
+         "        at[i] = pos;\n"
+         "        __threadfence_block();\n"
+         "        atomicExch(st + pos, 2u + i);\n"
+         "        return (int)i;\n"
+         "      }\n"
+         "    }\n"
+         "    if (v == key) {\n"
+         "      u32 s = gx_lds_acquire(st + pos), spins = 0;\n"
+         "      while (s == 0u) {\n"
+         "        if (++spins > (1u << 20)) { atomicExch(err, 1); return -2; }\n"
+         "        __nanosleep(16);\n"
+         "        s = gx_lds_acquire(st + pos);\n"
+         "      }\n"
+         "      return s == 0xffffffffu ? -1 : (int)s - 2;\n"
+         "    }\n"
+         "    pos = (pos + 1u) & (GXA_D - 1);\n"
+         "  }\n"
+         "  return -1;\n"
+         "}\n";
+  } else {
+    // the block's table: -1 when the probe finds no room, -2 after a wait gave up
+    o << "__device__ int gxa_find_smem(u32* st, u32* nm, u64* ks, const u64* kv, u32 kn, u64 h, int* err) {\n"
+         "  u32 pos = __umulhi((u32)h, (u32)GXA_S);\n"
+         "  for (int pr = 0; pr < GXA_PROBES; pr++) {\n"
+         "    u32 s = gx_lds_acquire(st + pos);\n"
+         "    if (s == 0u) {\n"
+         "      s = atomicCAS(st + pos, 0u, 1u);\n"
+         "      if (s == 0u) {\n";
+    write_keys(o, "ks", "GXA_S", "pos", "        ");
+    o << "        nm[pos] = kn;\n"
+         "        __threadfence_block();\n"
+         "        atomicExch(st + pos, 2u);\n"
+         "        return (int)pos;\n"
+         "      }\n"
+         "    }\n"
+         "    u32 spins = 0;\n"
+         "    while (s == 1u) {\n"
+         "      if (++spins > (1u << 20)) { atomicExch(err, 1); return -2; }\n"
+         "      __nanosleep(16);\n"
+         "      s = gx_lds_acquire(st + pos);\n"
+         "    }\n"
+         "    if (*(volatile u32*)(nm + pos) == kn && " << same_keys("ks", "GXA_S", "pos") << ") return (int)pos;\n"
+         "    pos = pos + 1u == GXA_S ? 0u : pos + 1u;\n"
+         "  }\n"
+         "  return -1;\n"
+         "}\n";
+    // the block's dictionary of groups with warp accumulators: the group's index,
+    // -1 when it has none and no room is left, -2 after a wait gave up
+    o << "__device__ int gxa_find_warp(u32* st, u32* nm, u64* ks, u32* at, u32* ng, const u64* kv, u32 kn, u64 h, int* err) {\n"
+         "  u32 pos = (u32)h & (GXA_D - 1);\n"
+         "  for (int pr = 0; pr < GXA_D; pr++) {\n"
+         "    u32 s = gx_lds_acquire(st + pos);\n"
+         "    if (s == 0u) {\n"
+         "      if (*(volatile u32*)ng >= GXA_G) return -1;\n"
+         "      s = atomicCAS(st + pos, 0u, 1u);\n"
+         "      if (s == 0u) {\n"
+         "        const u32 i = atomicAdd(ng, 1u);\n"
+         "        if (i >= GXA_G) { atomicExch(st + pos, 0xffffffffu); return -1; }\n";  // lost the last place
+    write_keys(o, "ks", "GXA_D", "pos", "        ");
+    o << "        nm[pos] = kn; at[i] = pos;\n"
+         "        __threadfence_block();\n"
+         "        atomicExch(st + pos, 2u + i);\n"
+         "        return (int)i;\n"
+         "      }\n"
+         "    }\n"
+         "    u32 spins = 0;\n"
+         "    while (s == 1u) {\n"
+         "      if (++spins > (1u << 20)) { atomicExch(err, 1); return -2; }\n"
+         "      __nanosleep(16);\n"
+         "      s = gx_lds_acquire(st + pos);\n"
+         "    }\n"
+         "    if (s != 0xffffffffu && *(volatile u32*)(nm + pos) == kn && " << same_keys("ks", "GXA_D", "pos") << ") return (int)s - 2;\n"
+         "    pos = (pos + 1u) & (GXA_D - 1);\n"
+         "  }\n"
+         "  return -1;\n"
+         "}\n";
+  }
   // the global table: -1 when the whole table was probed (overflow) or a wait gave up
   o << "__device__ long long gxa_find_global(const GxAggArgs& g, const u64* kv, u32 kn, u64 h) {\n"
        "  u64 pos = h & (g.cap - 1ull);\n"
@@ -2832,11 +2911,16 @@ std::string generate_agg_kernel(const Plan& p, const AggLayout& L, const KernelC
   o << "  u64* const d_ks_ = (u64*)gx_smem; u64* const d_gs_ = d_ks_ + GXA_NK * GXA_D;\n";
   o << "  u32* const d_st_ = (u32*)(d_gs_ + GXA_D); u32* const d_nm_ = d_st_ + GXA_D; u32* const d_at_ = d_nm_ + GXA_D;\n";
   o << "  u64* const s_warp_ = (u64*)(gx_smem + " << sh.dict_bytes << ");\n";
-  o << "  u64* const s_ks_ = s_warp_; u64* const s_acc_ = s_ks_ + GXA_NK * GXA_S;\n";
-  o << "  u32* const s_st_ = (u32*)(s_acc_ + " << sh.accs << " * GXA_S); u32* const s_nm_ = s_st_ + GXA_S;\n";
-  o << "  u32* const s_rows_ = s_nm_ + GXA_S; u32* const s_cnt_ = s_rows_ + GXA_S;\n";
+  if (sh.packed) {
+    o << "  u64* const s_pk_ = s_warp_; u64* const s_acc_ = s_pk_ + GXA_S;\n";
+    o << "  u32* const s_rows_ = (u32*)(s_acc_ + " << sh.accs << " * GXA_S); u32* const s_cnt_ = s_rows_ + GXA_S;\n";
+  } else {
+    o << "  u64* const s_ks_ = s_warp_; u64* const s_acc_ = s_ks_ + GXA_NK * GXA_S;\n";
+    o << "  u32* const s_st_ = (u32*)(s_acc_ + " << sh.accs << " * GXA_S); u32* const s_nm_ = s_st_ + GXA_S;\n";
+    o << "  u32* const s_rows_ = s_nm_ + GXA_S; u32* const s_cnt_ = s_rows_ + GXA_S;\n";
+  }
   o << "  int mode_ = GXA_G > 0 ? 1 : 2;\n";
-  o << "  for (int i = threadIdx.x; i < GXA_D; i += blockDim.x) d_st_[i] = 0u;\n";
+  o << "  for (int i = threadIdx.x; i < GXA_D; i += blockDim.x) { d_st_[i] = 0u;" << (sh.packed ? " d_ks_[i] = 0ull;" : "") << " }\n";
   o << "  if (threadIdx.x == 0) { s_ng_ = 0u; s_over_ = 0; }\n";
   o << "  if (mode_ == 1) {\n";
   o << "    for (int i = threadIdx.x; i < GX_WARPS * GXA_GR; i += blockDim.x) {\n";
@@ -2848,7 +2932,7 @@ std::string generate_agg_kernel(const Plan& p, const AggLayout& L, const KernelC
   o << "    }\n  }\n";
   o << "  auto table_init_ = [&]() {\n";
   o << "    for (int i = threadIdx.x; i < GXA_S; i += blockDim.x) {\n";
-  o << "      s_st_[i] = 0u; s_rows_[i] = 0u;\n";
+  o << "      " << (sh.packed ? "s_pk_[i] = 0ull" : "s_st_[i] = 0u") << "; s_rows_[i] = 0u;\n";
   for (int j = 0; j < na; j++) {
     if (sh.acc_slot[j] >= 0) o << "      s_acc_[" << sh.acc_slot[j] << " * GXA_S + i] = " << agg_identity(L.kinds[j], false) << ";\n";
     if (sh.cnt_slot[j] >= 0) o << "      s_cnt_[" << sh.cnt_slot[j] << " * GXA_S + i] = 0u;\n";
@@ -2898,7 +2982,7 @@ std::string generate_agg_kernel(const Plan& p, const AggLayout& L, const KernelC
     o << in2 << "kv[" << j << "] = " << g.V(id) << " ? (u64)(" << g.B(id) << ") : 0ull; if (!(" << g.V(id)
       << ")) kn_ |= " << (1u << j) << "u;\n";
   }
-  o << in2 << "const u64 h_ = gxa_hash(kv, kn_);\n";
+  o << in2 << (sh.packed ? "const u64 pk_ = gxa_pack(kv, kn_);\n" : "const u64 h_ = gxa_hash(kv, kn_);\n");
   for (int j = 0; j < na; j++) {
     const int in = L.in_nodes[j];
     o << in2 << "const bool ok" << j << "_ = " << (in >= 0 ? g.V(in) : std::string("true")) << ";\n";
@@ -2907,8 +2991,11 @@ std::string generate_agg_kernel(const Plan& p, const AggLayout& L, const KernelC
   auto in_ = [](int j) { return "in" + std::to_string(j) + "_"; };
   auto ok_ = [](int j) { return "ok" + std::to_string(j) + "_"; };
   o << in2 << "int sl_ = -3;\n";
-  o << in2 << "if (act) sl_ = mode_ == 1 ? gxa_find_warp(d_st_, d_nm_, d_ks_, d_at_, &s_ng_, kv, kn_, h_, ga.err)\n"
-    << in2 << "                          : gxa_find_smem(s_st_, s_nm_, s_ks_, kv, kn_, h_, ga.err);\n";
+  if (sh.packed)
+    o << in2 << "if (act) sl_ = mode_ == 1 ? gxa_find_dict(d_st_, d_ks_, d_at_, &s_ng_, pk_, ga.err) : gxa_find_table(s_pk_, pk_);\n";
+  else
+    o << in2 << "if (act) sl_ = mode_ == 1 ? gxa_find_warp(d_st_, d_nm_, d_ks_, d_at_, &s_ng_, kv, kn_, h_, ga.err)\n"
+      << in2 << "                          : gxa_find_smem(s_st_, s_nm_, s_ks_, kv, kn_, h_, ga.err);\n";
   // a group without warp accumulators: the round is left for the table
   o << in2 << "if (mode_ == 1 && __any_sync(GX_FULL, sl_ == -1 || *(volatile int*)&s_over_ != 0)) {\n";
   o << in2 << "  *(volatile int*)&s_over_ = 1; skip_ = base_; full_ = true;\n";
@@ -2997,7 +3084,7 @@ std::string generate_agg_kernel(const Plan& p, const AggLayout& L, const KernelC
   o << in2 << "}\n";
   // rows whose group found no room in the block go to the global table
   o << in2 << "if (mode_ == 2 && act && sl_ == -1) {\n";
-  o << in2 << "  const long long gs_ = gxa_find_global(ga, kv, kn_, h_);\n";
+  o << in2 << "  const long long gs_ = gxa_find_global(ga, kv, kn_, " << (sh.packed ? "gxa_hash(kv, kn_)" : "h_") << ");\n";
   o << in2 << "  if (gs_ >= 0) {\n";
   o << in2 << "    atomicAdd((unsigned long long*)(ga.rows + gs_), 1ull);\n";
   for (int j = 0; j < na; j++) {
@@ -3026,8 +3113,13 @@ std::string generate_agg_kernel(const Plan& p, const AggLayout& L, const KernelC
   o << "      for (int w = 0; w < GX_WARPS; w++)\n        for (int r = 0; r < GXA_R; r++)\n"
        "          rows_ += s_warp_[" << sh.rows_cell << " * GXA_CS + w * GXA_GR + (int)threadIdx.x * GXA_R + r];\n";
   o << "      u64 kv[GXA_NK]; kv[0] = 0ull;\n";
-  for (int j = 0; j < nk; j++) o << "      kv[" << j << "] = d_ks_[" << j << " * GXA_D + i];\n";
-  o << "      d_gs_[threadIdx.x] = rows_ ? (u64)gxa_find_global(ga, kv, d_nm_[i], gxa_hash(kv, d_nm_[i])) : ~0ull;\n";
+  if (sh.packed) {
+    o << "      const u32 kn_ = gxa_unpack(d_ks_[i], kv);\n";
+  } else {
+    for (int j = 0; j < nk; j++) o << "      kv[" << j << "] = d_ks_[" << j << " * GXA_D + i];\n";
+    o << "      const u32 kn_ = d_nm_[i];\n";
+  }
+  o << "      d_gs_[threadIdx.x] = rows_ ? (u64)gxa_find_global(ga, kv, kn_, gxa_hash(kv, kn_)) : ~0ull;\n";
   o << "    }\n";
   o << "    __syncthreads();\n";
   // one warp per group and cell: lane w takes warp w's replicas, then a tree over lanes
@@ -3054,10 +3146,14 @@ std::string generate_agg_kernel(const Plan& p, const AggLayout& L, const KernelC
   }
   o << "  } else {\n";
   o << "    for (int i = threadIdx.x; i < GXA_S; i += blockDim.x) {\n";
-  o << "      if (s_st_[i] != 2u || s_rows_[i] == 0u) continue;\n";
+  o << "      if (s_rows_[i] == 0u" << (sh.packed ? "" : " || s_st_[i] != 2u") << ") continue;\n";
   o << "      u64 kv[GXA_NK]; kv[0] = 0ull;\n";
-  for (int j = 0; j < nk; j++) o << "      kv[" << j << "] = s_ks_[" << j << " * GXA_S + i];\n";
-  o << "      const u32 kn_ = s_nm_[i];\n";
+  if (sh.packed) {
+    o << "      const u32 kn_ = gxa_unpack(s_pk_[i], kv);\n";
+  } else {
+    for (int j = 0; j < nk; j++) o << "      kv[" << j << "] = s_ks_[" << j << " * GXA_S + i];\n";
+    o << "      const u32 kn_ = s_nm_[i];\n";
+  }
   o << "      const long long gs_ = gxa_find_global(ga, kv, kn_, gxa_hash(kv, kn_));\n";
   o << "      if (gs_ < 0) continue;\n";
   o << "      atomicAdd((unsigned long long*)(ga.rows + gs_), (unsigned long long)s_rows_[i]);\n";

@@ -132,6 +132,7 @@ constexpr int kAggDict = 64;
 struct AggShared {
   int warp_groups = 0, replicas = 1, cells = 0, rows_cell = 0;
   int slots = 0, accs = 0;
+  bool packed = false;  // a group's keys are one word
   int dict_bytes = 0, dyn_bytes = 0;
   std::vector<int> acc_cell, cnt_cell, acc_slot, cnt_slot;
 };
