@@ -240,6 +240,10 @@ __device__ __forceinline__ void gx_bulk_g2s(void* dst, const void* src, u32 byte
                "l"(src), "r"(bytes), "r"(gx_saddr(bar))
                : "memory");
 }
+// brings `bytes` (a multiple of 16) from p's 16-byte block on into L2
+__device__ __forceinline__ void gx_prefetch_l2(const void* p, u32 bytes) {
+  asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"((unsigned long long)p & ~15ull), "r"(bytes) : "memory");
+}
 // 16-byte asynchronous global -> shared copy (L2 only), and an arrival on an
 // mbarrier once every earlier copy of this thread has landed
 __device__ __forceinline__ void gx_cp16(void* dst, const void* src) {

@@ -2967,6 +2967,29 @@ std::string generate_agg_kernel(const Plan& p, const AggLayout& L, const KernelC
   o << "    unsigned short* const kl_ = s_kept_[warp];\n";
   emit_kept_list(o, "bal", "kl_", "total_", "    ");
   o << "    __syncwarp();\n";
+  {
+    std::vector<int> cols;
+    for (const auto& ids : {pred_ids, row_ids})
+      for (int id : ids)
+        if (p.nodes[id].kind == Node::COL && std::find(cols.begin(), cols.end(), p.nodes[id].col) == cols.end())
+          cols.push_back(p.nodes[id].col);
+    // The next chunk's columns are brought into L2 while this one's rows are
+    // combined: with 32 warps on an SM (one block, whose tables fill its shared
+    // memory) a round mostly waits for its loads.  Lane i takes column i; not for
+    // a chunk of which less than a quarter is kept, where most bytes would go
+    // unread.  Kernel us without and with: 2557 dates 340 / 332, two flag columns
+    // at 2^26 rows 1270 / 1243.
+    if (!cols.empty() && cols.size() <= 32) {
+      o << "    {\n      const i64 nx_ = (i64)__shfl_sync(GX_FULL, tk_, 0);\n";
+      o << "      if (total_ >= GX_V * 8u && (nx_ + 1) * (GX_V * 32) <= a.n) {\n";
+      o << "        const char* q_ = nullptr; u32 w_ = 0u;\n";
+      for (size_t i = 0; i < cols.size(); i++)
+        o << "        if (lane == " << i << ") { q_ = (const char*)a.in_data[" << cols[i] << "]; w_ = "
+          << type_size(p.schema[cols[i]]) << "u; }\n";
+      o << "        if (w_) gx_prefetch_l2(q_ + nx_ * (i64)(GX_V * 32u * w_), GX_V * 32u * w_);\n";
+      o << "      }\n    }\n";
+    }
+  }
   g.masks_ = Gen::Masks::KEPT;
   g.emit_mask_words(o, row_ids, {}, "    ");
   o << "    full_ = false;\n";
