@@ -2405,9 +2405,35 @@ std::vector<int> conjunct_columns(const Plan& p, int c) {
 // cost the same either way (1.88 ms), its aggregation 1.48 ms against 1.64 ms.
 int auto_native_f64_ops() { return kNativeAddSub | kNativeMul; }
 
+// Projection kernels wait for memory, so one more block of warps per SM is worth
+// more than the compiler's last registers: five outputs over five columns, 2^25
+// rows, 88 registers 499 us, capped at 80 474 (72 477, 64 478, 56 513 with spills).
+// Held to the cap are plans whose loads of a warp's words leave half of it and that
+// call no transcendental function (those keep polynomials and the call's own
+// state live).
+constexpr int kProjectRegs = 80;
+static bool project_fits_cap(const Plan& p, const KernelConfig& cfg) {
+  std::set<int> seen;
+  int regs = 0;
+  bool fits = true;
+  std::function<void(int)> go = [&](int id) {
+    if (id < 0 || !seen.insert(id).second) return;
+    const Node& n = p.nodes[id];
+    if (n.kind == Node::COL) regs += cfg.words * std::max(1, type_size(p.schema[n.col]) / 4);
+    if (n.kind != Node::OP) return;
+    fits = fits && Gen::op_cost(n.op) < 64;
+    go(n.a);
+    go(n.b);
+  };
+  for (const auto& o : p.outputs)
+    if (o.kind == OutSpec::NODE) go(o.node);
+  return fits && regs <= kProjectRegs / 2;
+}
+
 std::string generate_kernel(const Plan& p, KernelKind kind, const KernelConfig& cfg_in, const std::string& name) {
   KernelConfig cfg = cfg_in;
   if (cfg.native_f64_ops < 0) cfg.native_f64_ops = auto_native_f64_ops();
+  if (kind == KernelKind::PROJECT && cfg.max_regs == 0 && project_fits_cap(p, cfg)) cfg.max_regs = kProjectRegs;
   Gen g(p, cfg);
   if (p.has_filter() && cfg.dense) {
     // columns whose data the predicate reads (not only their validity, as
