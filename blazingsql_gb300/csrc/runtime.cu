@@ -346,9 +346,15 @@ __global__ void k_fill_mask(uint32_t* dst, int64_t nrows, bool valid, int64_t ds
   }
 }
 
-// Exclusive scan of per-tile counts in place (one CTA of 1024 threads walks
-// the array in chunks); *total receives the sum.
-__global__ void __launch_bounds__(1024) k_scan_tiles(uint64_t* counts, int64_t n, unsigned long long* total) {
+// Exclusive scans of per-tile counts in place (one CTA of 1024 threads walks an
+// array in chunks); *total receives an array's sum.
+struct ScanTasks {
+  ScanTask task[kScanTasks];
+};
+__global__ void __launch_bounds__(1024) k_scan_tiles(ScanTasks ts) {
+  uint64_t* const counts = ts.task[blockIdx.x].counts;
+  const int64_t n = ts.task[blockIdx.x].n;
+  unsigned long long* const total = ts.task[blockIdx.x].total;
   __shared__ uint64_t s_warp[32];
   __shared__ uint64_t s_carry;
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
@@ -454,10 +460,15 @@ void launch_fill_mask(uint32_t* dst, int64_t nrows, bool valid, int64_t dst_word
   check_cuda(cudaGetLastError(), "k_fill_mask launch");
 }
 
-void launch_scan_tiles(uint64_t* counts, int64_t n, unsigned long long* total, cudaStream_t s) {
-  k_scan_tiles<<<1, 1024, 0, s>>>(counts, n, total);
-  g_launches.fetch_add(1);
-  check_cuda(cudaGetLastError(), "k_scan_tiles launch");
+void launch_scan_tiles(const std::vector<ScanTask>& tasks, cudaStream_t s) {
+  for (size_t at = 0; at < tasks.size(); at += kScanTasks) {
+    const size_t k = std::min<size_t>(tasks.size() - at, kScanTasks);
+    ScanTasks ts{};
+    std::copy_n(tasks.begin() + at, k, ts.task);
+    k_scan_tiles<<<(unsigned)k, 1024, 0, s>>>(ts);
+    g_launches.fetch_add(1);
+    check_cuda(cudaGetLastError(), "k_scan_tiles launch");
+  }
 }
 
 // ------------------------------------------------------------ plan execution
@@ -746,7 +757,7 @@ void CompiledPlan::enqueue_filter(const std::vector<ColumnView>& cols, gx_column
     int64_t grid = (int64_t)device_sm_count() * kc.max_blocks_per_sm;
     if (grid > ntiles) grid = ntiles;
     launch(kc, (int)grid, s, a, true);
-    launch_scan_tiles(tile_status, ntiles, hdr + 3, s);
+    launch_scan_tiles({{tile_status, ntiles, hdr + 3}}, s);
   }
   const JitKernel k = kernel(two_pass ? KernelKind::WRITE_FILTER : KernelKind::FUSED_FILTER, nb);
   int64_t grid = (int64_t)device_sm_count() * k.max_blocks_per_sm;
@@ -900,7 +911,7 @@ void CompiledPlan::run_filter(const std::vector<ColumnView>& cols, gx_column* ou
       int64_t grid = (int64_t)device_sm_count() * kc.max_blocks_per_sm;
       if (grid > ntiles) grid = ntiles;
       launch(kc, (int)grid, s, a, true);
-      launch_scan_tiles(status, ntiles, hdr + 3, s);
+      launch_scan_tiles({{status, ntiles, hdr + 3}}, s);
       if (extras && extras->conj_counts && extras->conj_counts_host)
         check_cuda(cudaMemcpyAsync(extras->conj_counts_host, extras->conj_counts, 16 * 8, cudaMemcpyDeviceToHost, s),
                    "conjunct counts readback");

@@ -200,7 +200,14 @@ void launch_copy_mask(const uint32_t* src, int64_t src_bit, uint32_t* dst, int64
                       cudaStream_t s);
 void launch_fill(void* dst, int width, uint64_t value, int64_t n, cudaStream_t s);
 void launch_fill_mask(uint32_t* dst, int64_t nrows, bool valid, int64_t dst_words, cudaStream_t s);
-void launch_scan_tiles(uint64_t* counts, int64_t n, unsigned long long* total, cudaStream_t s);
+// Exclusive scans in place, a block each, kScanTasks per launch.
+struct ScanTask {
+  uint64_t* counts;
+  int64_t n;
+  unsigned long long* total;
+};
+constexpr int kScanTasks = 32;
+void launch_scan_tiles(const std::vector<ScanTask>& tasks, cudaStream_t s);
 // launches a plan kernel with an arbitrary parameter list (counted, optionally timed)
 void launch_raw(const JitKernel& k, int grid, cudaStream_t s, void** params, bool timed);
 

@@ -1489,7 +1489,8 @@ struct Build {
   BuildArgs b{};
   XformArgs x{};
   unsigned nblocks = 0;
-  const volatile unsigned long long* total = nullptr;  // the character total, once the sizes are scanned
+  uint64_t* sums = nullptr;  // the blocks' character totals, then their starts
+  unsigned long long* total = nullptr;  // the character total, once the sizes are scanned
 };
 }  // namespace
 
@@ -1582,15 +1583,14 @@ static void with_class(XformClass c, F&& f) {
   }
 }
 
-// the sizing launch and the scan of the block totals
 static void launch_sizes(Build& b, uint64_t* sums, unsigned long long* total, int64_t rows, cudaStream_t s) {
   *total = 0;
   b.total = total;
+  b.sums = sums;
   if (rows == 0) return;
   if (b.xform) with_class(b.cls, [&](auto c) { k_xf_sizes<decltype(c)::value><<<b.nblocks, kBuildWarps * 32, 0, s>>>(b.x); });
   else k_str_sizes<<<b.nblocks, kBuildWarps * 32, 0, s>>>(b.b);
   check_cuda(cudaGetLastError(), "string sizes");
-  launch_scan_tiles(sums, b.nblocks, total, s);
   add_launches(1);
 }
 
@@ -1682,6 +1682,10 @@ void StringBuilds::transform(const StringOp& op, const StrSource& a, const StrSo
 std::vector<gx_column> StringBuilds::finish() {
   std::vector<gx_column> out;
   if (st_->builds.empty()) return out;
+  std::vector<ScanTask> scans;  // of the block totals
+  for (auto& b : st_->builds)
+    if (b.out.size > 0) scans.push_back({b.sums, b.nblocks, b.total});
+  launch_scan_tiles(scans, s_);
   check_cuda(cudaStreamSynchronize(s_), "string size sync");
   for (auto& b : st_->builds) {
     const uint64_t total = *b.total;
