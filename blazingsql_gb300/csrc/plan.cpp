@@ -2598,11 +2598,16 @@ std::string generate_kernel(const Plan& p, KernelKind kind, const KernelConfig& 
 //    each of the first warp_groups groups the block meets, `replicas` of each, so
 //    that as many lanes of one group update them side by side: a load, one
 //    operation and a store per accumulator, no combining and no atomic, repeated
-//    while a round holds more lanes of a group (two passes for six groups and five
-//    replicas).  Rounds with more than three passes' worth combine over a tree
-//    within the warp first.  The tree alone took 280 of 640 instructions per 32
-//    rows and five FP64 instructions per sum, the passes take about 90 and two:
-//    order-line rows by two flags, nine aggregations, 2^26 rows: 1.48 -> 1.30 ms.
+//    while a round holds more lanes of a group.  Rounds with more than three
+//    passes' worth combine over a tree within the warp first.  The tree alone took
+//    280 of 640 instructions per 32 rows and five FP64 instructions per sum, the
+//    passes take about 90 and two: order-line rows by two flags (four groups, nine
+//    aggregations), 2^26 rows: 1.48 -> 1.30 ms.  The room goes to 8 or
+//    more groups with up to 16 replicas first, so that a round's largest group
+//    mostly takes one pass (four groups, 6 / 9 / 12 / 16 replicas: 1362 / 1246 /
+//    1229 / 1126 us).  A block that meets more groups merges what it has and goes
+//    on with half the replicas for twice the groups, unless 32 of its rows held
+//    more than those; 1142 us with both splits.
 // 2. Many groups.  When a group finds no room there, the block's warps finish
 //    their chunks, the warps' accumulators go to the global table, and the block
 //    goes on with one hash table in the same shared memory (thousands of groups),
@@ -2669,11 +2674,14 @@ AggShared agg_shared(const Plan& p, const AggLayout& L, const KernelConfig& cfg)
   s.dict_bytes = (kAggDict * (8 * (nk + 1) + 12) + 15) / 16 * 16;
   const int budget = L.smem_bytes - s.dict_bytes;
   const int room = budget / (cfg.warps * s.cells * 8);  // words of a cell per warp
-  s.replicas = std::max(1, std::min(8, room / 16));
+  s.replicas = std::max(1, std::min(16, room / 8));
   s.warp_groups = std::min(kAggDict / 2, room / s.replicas);
+  s.replicas2 = std::max(1, std::min(8, room / 16));
+  s.warp_groups2 = std::min(kAggDict / 2, room / s.replicas2);
+  s.cell_words = std::max(s.warp_groups * s.replicas, s.warp_groups2 * s.replicas2);
   const int slot_bytes = 8 * ((s.packed ? 1 : nk) + s.accs) + 4 * ((s.packed ? 1 : 3) + cnts);
   s.slots = std::max(16, std::min(8192, budget / slot_bytes) / 8 * 8);
-  s.dyn_bytes = s.dict_bytes + std::max(s.warp_groups * s.replicas * cfg.warps * s.cells * 8, s.slots * slot_bytes);
+  s.dyn_bytes = s.dict_bytes + std::max(s.cell_words * cfg.warps * s.cells * 8, s.slots * slot_bytes);
   return s;
 }
 
@@ -2691,7 +2699,9 @@ std::string generate_agg_kernel(const Plan& p, const AggLayout& L, const KernelC
   const int nk = (int)L.key_nodes.size(), na = (int)L.kinds.size();
   const uint64_t rows_cnt = agg_counts_are_rows(p, L);
   const AggShared sh = agg_shared(p, L, cfg);
-  o << "#define GXA_S " << sh.slots << "\n#define GXA_G " << sh.warp_groups << "\n#define GXA_R " << sh.replicas << "\n#define GXA_D " << kAggDict
+  const bool two = sh.warp_groups2 > sh.warp_groups;  // a second split of the warps' accumulators holds more groups
+  o << "#define GXA_S " << sh.slots << "\n#define GXA_G " << sh.warp_groups << "\n#define GXA_R " << sh.replicas << "\n#define GXA_G2 "
+    << sh.warp_groups2 << "\n#define GXA_R2 " << sh.replicas2 << "\n#define GXA_D " << kAggDict
     << "\n#define GXA_NK " << std::max(nk, 1) << "\n#define GXA_PROBES 32\n";
   // key hash (null keys hash as zero with their null bit set)
   // (32-bit multiplies by odd constants, a key's high half only where it has
@@ -2749,16 +2759,16 @@ std::string generate_agg_kernel(const Plan& p, const AggLayout& L, const KernelC
          "  }\n"
          "  return -1;\n"
          "}\n";
-    o << "__device__ int gxa_find_dict(u32* st, u64* pk, u32* at, u32* ng, u64 key, int* err) {\n"
+    o << "__device__ int gxa_find_dict(u32* st, u64* pk, u32* at, u32* ng, const u32* room, u64 key, int* err) {\n"
          "  u32 pos = __umulhi(gxa_place(key), (u32)GXA_D);\n"
          "  for (int pr = 0; pr < GXA_D; pr++) {\n"
          "    u64 v = *(volatile u64*)(pk + pos);\n"
          "    if (v == 0ull) {\n"
-         "      if (*(volatile u32*)ng >= GXA_G) return -1;\n"
+         "      if (*(volatile u32*)ng >= *(volatile const u32*)room) return -1;\n"
          "      v = atomicCAS((unsigned long long*)(pk + pos), 0ull, (unsigned long long)key);\n"
          "      if (v == 0ull) {\n"
          "        const u32 i = atomicAdd(ng, 1u);\n"
-         "        if (i >= GXA_G) { atomicExch(st + pos, 0xffffffffu); return -1; }\n"  // lost the last place
+         "        if (i >= *(volatile const u32*)room) { atomicExch(st + pos, 0xffffffffu); return -1; }\n"  // lost the last place
          "        at[i] = pos;\n"
          "        __threadfence_block();\n"
          "        atomicExch(st + pos, 2u + i);\n"
@@ -2807,16 +2817,16 @@ std::string generate_agg_kernel(const Plan& p, const AggLayout& L, const KernelC
          "}\n";
     // the block's dictionary of groups with warp accumulators: the group's index,
     // -1 when it has none and no room is left, -2 after a wait gave up
-    o << "__device__ int gxa_find_warp(u32* st, u32* nm, u64* ks, u32* at, u32* ng, const u64* kv, u32 kn, u64 h, int* err) {\n"
+    o << "__device__ int gxa_find_warp(u32* st, u32* nm, u64* ks, u32* at, u32* ng, const u32* room, const u64* kv, u32 kn, u64 h, int* err) {\n"
          "  u32 pos = (u32)h & (GXA_D - 1);\n"
          "  for (int pr = 0; pr < GXA_D; pr++) {\n"
          "    u32 s = gx_lds_acquire(st + pos);\n"
          "    if (s == 0u) {\n"
-         "      if (*(volatile u32*)ng >= GXA_G) return -1;\n"
+         "      if (*(volatile u32*)ng >= *(volatile const u32*)room) return -1;\n"
          "      s = atomicCAS(st + pos, 0u, 1u);\n"
          "      if (s == 0u) {\n"
          "        const u32 i = atomicAdd(ng, 1u);\n"
-         "        if (i >= GXA_G) { atomicExch(st + pos, 0xffffffffu); return -1; }\n";  // lost the last place
+         "        if (i >= *(volatile const u32*)room) { atomicExch(st + pos, 0xffffffffu); return -1; }\n";  // lost the last place
     write_keys(o, "ks", "GXA_D", "pos", "        ");
     o << "        nm[pos] = kn; at[i] = pos;\n"
          "        __threadfence_block();\n"
@@ -2930,7 +2940,7 @@ std::string generate_agg_kernel(const Plan& p, const AggLayout& L, const KernelC
   o << "  const i64 nwords = (a.n + 31) >> 5;\n";
   // ---- shared memory: the dictionary, then the warps' accumulators or the table
   // a cell: one 8-byte word per warp, group and replica, cell after cell
-  o << "#define GXA_GR (GXA_G * GXA_R)\n#define GXA_CS (GX_WARPS * GXA_GR)\n";
+  o << "#define GXA_GR " << sh.cell_words << "\n#define GXA_CS (GX_WARPS * GXA_GR)\n";
   o << "  const i64 nchunks = (nwords + GX_V - 1) / GX_V;\n";
   o << "  __shared__ unsigned short s_kept_[GX_WARPS][GX_V * 32];\n";
   o << "  __shared__ u32 s_ng_; __shared__ int s_over_;\n";
@@ -2946,8 +2956,13 @@ std::string generate_agg_kernel(const Plan& p, const AggLayout& L, const KernelC
     o << "  u32* const s_rows_ = s_nm_ + GXA_S; u32* const s_cnt_ = s_rows_ + GXA_S;\n";
   }
   o << "  int mode_ = GXA_G > 0 ? 1 : 2;\n";
+  // the split in use, groups and replicas of each (shared: it takes no register)
+  o << "  __shared__ u32 s_room_; __shared__ int s_rep_;\n";
+  o << "  if (threadIdx.x == 0) { s_room_ = GXA_G; s_rep_ = GXA_R; }\n";
+  if (two) o << "  __shared__ int s_many_;\n";
+  o << "  auto warps_init_ = [&]() {\n";
   o << "  for (int i = threadIdx.x; i < GXA_D; i += blockDim.x) { d_st_[i] = 0u;" << (sh.packed ? " d_ks_[i] = 0ull;" : "") << " }\n";
-  o << "  if (threadIdx.x == 0) { s_ng_ = 0u; s_over_ = 0; }\n";
+  o << "  if (threadIdx.x == 0) { s_ng_ = 0u; s_over_ = 0;" << (two ? " s_many_ = 0;" : "") << " }\n";
   o << "  if (mode_ == 1) {\n";
   o << "    for (int i = threadIdx.x; i < GX_WARPS * GXA_GR; i += blockDim.x) {\n";
   for (int j = 0; j < na; j++) {
@@ -2955,7 +2970,7 @@ std::string generate_agg_kernel(const Plan& p, const AggLayout& L, const KernelC
     if (sh.cnt_cell[j] >= 0) o << "      s_warp_[" << sh.cnt_cell[j] << " * GXA_CS + i] = 0ull;\n";
   }
   o << "      s_warp_[" << sh.rows_cell << " * GXA_CS + i] = 0ull;\n";
-  o << "    }\n  }\n";
+  o << "    }\n  }\n  };\n  warps_init_();\n";
   o << "  auto table_init_ = [&]() {\n";
   o << "    for (int i = threadIdx.x; i < GXA_S; i += blockDim.x) {\n";
   o << "      " << (sh.packed ? "s_pk_[i] = 0ull" : "s_st_[i] = 0u") << "; s_rows_[i] = 0u;\n";
@@ -3041,13 +3056,17 @@ std::string generate_agg_kernel(const Plan& p, const AggLayout& L, const KernelC
   auto ok_ = [](int j) { return "ok" + std::to_string(j) + "_"; };
   o << in2 << "int sl_ = -3;\n";
   if (sh.packed)
-    o << in2 << "if (act) sl_ = mode_ == 1 ? gxa_find_dict(d_st_, d_ks_, d_at_, &s_ng_, pk_, ga.err) : gxa_find_table(s_pk_, pk_);\n";
+    o << in2 << "if (act) sl_ = mode_ == 1 ? gxa_find_dict(d_st_, d_ks_, d_at_, &s_ng_, &s_room_, pk_, ga.err) : gxa_find_table(s_pk_, pk_);\n";
   else
-    o << in2 << "if (act) sl_ = mode_ == 1 ? gxa_find_warp(d_st_, d_nm_, d_ks_, d_at_, &s_ng_, kv, kn_, h_, ga.err)\n"
+    o << in2 << "if (act) sl_ = mode_ == 1 ? gxa_find_warp(d_st_, d_nm_, d_ks_, d_at_, &s_ng_, &s_room_, kv, kn_, h_, ga.err)\n"
       << in2 << "                          : gxa_find_smem(s_st_, s_nm_, s_ks_, kv, kn_, h_, ga.err);\n";
   // a group without warp accumulators: the round is left for the table
   o << in2 << "if (mode_ == 1 && __any_sync(GX_FULL, sl_ == -1 || *(volatile int*)&s_over_ != 0)) {\n";
   o << in2 << "  *(volatile int*)&s_over_ = 1; skip_ = base_; full_ = true;\n";
+  if (two) {  // more groups in these 32 rows than the second split holds: the table is next
+    o << in2 << "  const u32 same_ = __match_any_sync(GX_FULL, " << (sh.packed ? "pk_" : "h_") << ");\n";
+    o << in2 << "  if (__popc(__ballot_sync(GX_FULL, act && (same_ & ((1u << lane) - 1u)) == 0u)) > GXA_G2) *(volatile int*)&s_many_ = 1;\n";
+  }
   o << in2 << "  break;\n" << in2 << "}\n";
   o << in2 << "const bool sm_ = sl_ >= 0;\n";
   auto direct = [&](const std::string& ind) {
@@ -3080,11 +3099,12 @@ std::string generate_agg_kernel(const Plan& p, const AggLayout& L, const KernelC
       if (g2) o << ind << "}\n";
     }
   };
-  o << in2 << "if (mode_ == 1 && mx_ <= 3 * GXA_R) {\n";
+  o << in2 << "const int rep_ = " << (two ? "*(volatile int*)&s_rep_" : "GXA_R") << ";\n";
+  o << in2 << "if (mode_ == 1 && mx_ <= 3 * rep_) {\n";
   o << in2 << "  const int rank_ = __popc(peers_ & ((1u << lane) - 1u));\n";
-  o << in2 << "  for (int p_ = 0; p_ < mx_; p_ += GXA_R) {\n";
-  o << in2 << "    if (sm_ && (u32)(rank_ - p_) < (u32)GXA_R) {\n";
-  o << in2 << "      u64* const c_ = s_warp_ + warp * GXA_GR + sl_ * GXA_R + (rank_ - p_);\n";
+  o << in2 << "  for (int p_ = 0; p_ < mx_; p_ += rep_) {\n";
+  o << in2 << "    if (sm_ && (u32)(rank_ - p_) < (u32)rep_) {\n";
+  o << in2 << "      u64* const c_ = s_warp_ + warp * GXA_GR + sl_ * rep_ + (rank_ - p_);\n";
   update(in2 + "      ", "1ull", "", "in", true);
   o << in2 << "    }\n";
   o << in2 << "    __syncwarp();\n";  // the next pass's lanes update the same words
@@ -3115,7 +3135,7 @@ std::string generate_agg_kernel(const Plan& p, const AggLayout& L, const KernelC
     o << i4 << "}\n";
     o << i4 << "if (sm_ && pr_.rank == 0) {\n";
     o << i4 << "  if (mode_ == 1) {\n";
-    o << i4 << "    u64* const c_ = s_warp_ + warp * GXA_GR + sl_ * GXA_R;\n";
+    o << i4 << "    u64* const c_ = s_warp_ + warp * GXA_GR + sl_ * rep_;\n";
     update(i4 + "    ", "(u64)__popc(peers_)", "c", "x", false);
     o << i4 << "  } else {\n";
     o << i4 << "    atomicAdd(&s_rows_[sl_], (u32)__popc(peers_));\n";
@@ -3155,12 +3175,12 @@ std::string generate_agg_kernel(const Plan& p, const AggLayout& L, const KernelC
   o << "  __syncthreads();\n";
   // ---- merge into the global table
   o << "  if (mode_ == 1) {\n";
-  o << "    const int ng_ = (int)min(s_ng_, (u32)GXA_G);\n";
+  o << "    const int ng_ = (int)min(s_ng_, s_room_); const int rep_ = s_rep_;\n";
   o << "    if ((int)threadIdx.x < ng_) {\n";
   o << "      const u32 i = d_at_[threadIdx.x];\n";
   o << "      u64 rows_ = 0ull;\n";  // none: its only round was left for the table
-  o << "      for (int w = 0; w < GX_WARPS; w++)\n        for (int r = 0; r < GXA_R; r++)\n"
-       "          rows_ += s_warp_[" << sh.rows_cell << " * GXA_CS + w * GXA_GR + (int)threadIdx.x * GXA_R + r];\n";
+  o << "      for (int w = 0; w < GX_WARPS; w++)\n        for (int r = 0; r < rep_; r++)\n"
+       "          rows_ += s_warp_[" << sh.rows_cell << " * GXA_CS + w * GXA_GR + (int)threadIdx.x * rep_ + r];\n";
   o << "      u64 kv[GXA_NK]; kv[0] = 0ull;\n";
   if (sh.packed) {
     o << "      const u32 kn_ = gxa_unpack(d_ks_[i], kv);\n";
@@ -3177,8 +3197,8 @@ std::string generate_agg_kernel(const Plan& p, const AggLayout& L, const KernelC
     o << "    for (int gi = (warp + " << cell << ") % GX_WARPS; gi < ng_; gi += GX_WARPS) {\n";
     o << "      const long long gs_ = (long long)d_gs_[gi];\n";
     o << "      " << ty << " x = " << id << ";\n";
-    o << "      if (lane < GX_WARPS) for (int r = 0; r < GXA_R; r++) { const " << ty << " y = *(const " << ty << "*)(s_warp_ + "
-      << cell << " * GXA_CS + lane * GXA_GR + gi * GXA_R + r); x = " << (comb == "+" ? "x + y" : comb + "(x, y)") << "; }\n";
+    o << "      if (lane < GX_WARPS) for (int r = 0; r < rep_; r++) { const " << ty << " y = *(const " << ty << "*)(s_warp_ + "
+      << cell << " * GXA_CS + lane * GXA_GR + gi * rep_ + r); x = " << (comb == "+" ? "x + y" : comb + "(x, y)") << "; }\n";
     o << "      #pragma unroll\n      for (int d = 16; d > 0; d >>= 1) { const " << ty
       << " y = __shfl_xor_sync(GX_FULL, x, d); x = " << (comb == "+" ? "x + y" : comb + "(x, y)") << "; }\n";
     o << "      if (lane == 0 && gs_ >= 0) " << store << "\n";
@@ -3219,9 +3239,16 @@ std::string generate_agg_kernel(const Plan& p, const AggLayout& L, const KernelC
   o << "    }\n";
   o << "  }\n";
   o << "  if (mode_ == 2 || s_over_ == 0) break;\n";
-  o << "  __syncthreads();\n";
-  o << "  mode_ = 2;\n";
-  o << "  table_init_();\n";
+  if (two) {
+    o << "  const bool again_ = s_room_ == GXA_G && s_many_ == 0;\n";
+    o << "  __syncthreads();\n";
+    o << "  if (again_) { if (threadIdx.x == 0) { s_room_ = GXA_G2; s_rep_ = GXA_R2; } warps_init_(); }\n";
+    o << "  else { mode_ = 2; table_init_(); }\n";
+  } else {
+    o << "  __syncthreads();\n";
+    o << "  mode_ = 2;\n";
+    o << "  table_init_();\n";
+  }
   o << "  __syncthreads();\n";
   o << "  }\n";
   o << "}\n";

@@ -131,6 +131,7 @@ std::string generate_agg_kernel(const Plan& plan, const AggLayout& L, const Kern
 constexpr int kAggDict = 64;
 struct AggShared {
   int warp_groups = 0, replicas = 1, cells = 0, rows_cell = 0;
+  int warp_groups2 = 0, replicas2 = 1, cell_words = 0;  // a second split, for more groups; words of a cell per warp
   int slots = 0, accs = 0;
   bool packed = false;  // a group's keys are one word
   int dict_bytes = 0, dyn_bytes = 0;
