@@ -2605,9 +2605,11 @@ std::string generate_kernel(const Plan& p, KernelKind kind, const KernelConfig& 
 //    aggregations), 2^26 rows: 1.48 -> 1.30 ms.  The room goes to 8 or
 //    more groups with up to 16 replicas first, so that a round's largest group
 //    mostly takes one pass (four groups, 6 / 9 / 12 / 16 replicas: 1362 / 1246 /
-//    1229 / 1126 us).  A block that meets more groups merges what it has and goes
-//    on with half the replicas for twice the groups, unless 32 of its rows held
-//    more than those; 1142 us with both splits.
+//    1229 / 1126 us; 1142 with the number read from shared memory).  A block that
+//    meets more groups merges what it has and goes on with half the replicas, or
+//    fewer, for more groups, down to one, unless 32 of its rows held more than 28:
+//    then there are hundreds.  2^24 rows, nine aggregations, call us with 18 / 30 /
+//    45 groups: 373 / 362 / 493; through the table 1018 / 907 and more.
 // 2. Many groups.  When a group finds no room there, the block's warps finish
 //    their chunks, the warps' accumulators go to the global table, and the block
 //    goes on with one hash table in the same shared memory (thousands of groups),
@@ -2675,10 +2677,8 @@ AggShared agg_shared(const Plan& p, const AggLayout& L, const KernelConfig& cfg)
   const int budget = L.smem_bytes - s.dict_bytes;
   const int room = budget / (cfg.warps * s.cells * 8);  // words of a cell per warp
   s.replicas = std::max(1, std::min(16, room / 8));
-  s.warp_groups = std::min(kAggDict / 2, room / s.replicas);
-  s.replicas2 = std::max(1, std::min(8, room / 16));
-  s.warp_groups2 = std::min(kAggDict / 2, room / s.replicas2);
-  s.cell_words = std::max(s.warp_groups * s.replicas, s.warp_groups2 * s.replicas2);
+  s.warp_groups = std::min(kAggGroups, room / s.replicas);
+  s.cell_words = std::min(room, s.replicas * kAggGroups);
   const int slot_bytes = 8 * ((s.packed ? 1 : nk) + s.accs) + 4 * ((s.packed ? 1 : 3) + cnts);
   s.slots = std::max(16, std::min(8192, budget / slot_bytes) / 8 * 8);
   s.dyn_bytes = s.dict_bytes + std::max(s.cell_words * cfg.warps * s.cells * 8, s.slots * slot_bytes);
@@ -2699,9 +2699,10 @@ std::string generate_agg_kernel(const Plan& p, const AggLayout& L, const KernelC
   const int nk = (int)L.key_nodes.size(), na = (int)L.kinds.size();
   const uint64_t rows_cnt = agg_counts_are_rows(p, L);
   const AggShared sh = agg_shared(p, L, cfg);
-  const bool two = sh.warp_groups2 > sh.warp_groups;  // a second split of the warps' accumulators holds more groups
-  o << "#define GXA_S " << sh.slots << "\n#define GXA_G " << sh.warp_groups << "\n#define GXA_R " << sh.replicas << "\n#define GXA_G2 "
-    << sh.warp_groups2 << "\n#define GXA_R2 " << sh.replicas2 << "\n#define GXA_D " << kAggDict
+  const bool two = sh.replicas > 1 && sh.warp_groups < kAggGroups;  // fewer replicas hold more groups
+  o << "#define GXA_S " << sh.slots << "\n#define GXA_G " << sh.warp_groups << "\n#define GXA_R " << sh.replicas << "\n#define GXA_GMAX "
+    << kAggGroups << "\n#define GXA_GMANY 28\n#define GXA_GR " << sh.cell_words << "\n#define GXA_CS (GX_WARPS * GXA_GR)\n"
+    << "#define GXA_D " << kAggDict
     << "\n#define GXA_NK " << std::max(nk, 1) << "\n#define GXA_PROBES 32\n";
   // key hash (null keys hash as zero with their null bit set)
   // (32-bit multiplies by odd constants, a key's high half only where it has
@@ -2726,6 +2727,14 @@ std::string generate_agg_kernel(const Plan& p, const AggLayout& L, const KernelC
     for (int j = 0; j < nk; j++)
       os << ind << ks << "[" << j << "ull * " << stride << " + " << pos << "] = kv[" << j << "];\n";
   };
+  if (two)
+    // the next split of the accumulators' room, when a block met `need` groups in
+    // 32 rows: fewer replicas, more groups (replicas 0: the table is next)
+    o << "__device__ __noinline__ void gxa_next_split(u32* room, int* rep, u32 need) {\n"
+         "  int r = *rep; u32 g = *room;\n"
+         "  while (r > 1 && (g == *room || g < need + need / 4u)) { r /= 2; g = min((u32)GXA_GMAX, (u32)GXA_GR / (u32)r); }\n"
+         "  if (g > *room && need <= GXA_GMANY) { *room = g; *rep = r; } else { *rep = 0; }\n"
+         "}\n";
   if (sh.packed) {
     // a group as one word, and back; its place in shared memory is the key times
     // 2^32 over the golden ratio (Knuth's multiplicative hashing): consecutive
@@ -2940,7 +2949,6 @@ std::string generate_agg_kernel(const Plan& p, const AggLayout& L, const KernelC
   o << "  const i64 nwords = (a.n + 31) >> 5;\n";
   // ---- shared memory: the dictionary, then the warps' accumulators or the table
   // a cell: one 8-byte word per warp, group and replica, cell after cell
-  o << "#define GXA_GR " << sh.cell_words << "\n#define GXA_CS (GX_WARPS * GXA_GR)\n";
   o << "  const i64 nchunks = (nwords + GX_V - 1) / GX_V;\n";
   o << "  __shared__ unsigned short s_kept_[GX_WARPS][GX_V * 32];\n";
   o << "  __shared__ u32 s_ng_; __shared__ int s_over_;\n";
@@ -2959,10 +2967,10 @@ std::string generate_agg_kernel(const Plan& p, const AggLayout& L, const KernelC
   // the split in use, groups and replicas of each (shared: it takes no register)
   o << "  __shared__ u32 s_room_; __shared__ int s_rep_;\n";
   o << "  if (threadIdx.x == 0) { s_room_ = GXA_G; s_rep_ = GXA_R; }\n";
-  if (two) o << "  __shared__ int s_many_;\n";
+  if (two) o << "  __shared__ u32 s_need_;\n";
   o << "  auto warps_init_ = [&]() {\n";
   o << "  for (int i = threadIdx.x; i < GXA_D; i += blockDim.x) { d_st_[i] = 0u;" << (sh.packed ? " d_ks_[i] = 0ull;" : "") << " }\n";
-  o << "  if (threadIdx.x == 0) { s_ng_ = 0u; s_over_ = 0;" << (two ? " s_many_ = 0;" : "") << " }\n";
+  o << "  if (threadIdx.x == 0) { s_ng_ = 0u; s_over_ = 0;" << (two ? " s_need_ = 0u;" : "") << " }\n";
   o << "  if (mode_ == 1) {\n";
   o << "    for (int i = threadIdx.x; i < GX_WARPS * GXA_GR; i += blockDim.x) {\n";
   for (int j = 0; j < na; j++) {
@@ -3063,9 +3071,10 @@ std::string generate_agg_kernel(const Plan& p, const AggLayout& L, const KernelC
   // a group without warp accumulators: the round is left for the table
   o << in2 << "if (mode_ == 1 && __any_sync(GX_FULL, sl_ == -1 || *(volatile int*)&s_over_ != 0)) {\n";
   o << in2 << "  *(volatile int*)&s_over_ = 1; skip_ = base_; full_ = true;\n";
-  if (two) {  // more groups in these 32 rows than the second split holds: the table is next
+  if (two) {  // the groups of these 32 rows tell how many there may be
     o << in2 << "  const u32 same_ = __match_any_sync(GX_FULL, " << (sh.packed ? "pk_" : "h_") << ");\n";
-    o << in2 << "  if (__popc(__ballot_sync(GX_FULL, act && (same_ & ((1u << lane) - 1u)) == 0u)) > GXA_G2) *(volatile int*)&s_many_ = 1;\n";
+    o << in2 << "  const u32 seen_ = (u32)__popc(__ballot_sync(GX_FULL, act && (same_ & ((1u << lane) - 1u)) == 0u));\n";
+    o << in2 << "  if (lane == 0) atomicMax(&s_need_, seen_);\n";
   }
   o << in2 << "  break;\n" << in2 << "}\n";
   o << in2 << "const bool sm_ = sl_ >= 0;\n";
@@ -3240,9 +3249,10 @@ std::string generate_agg_kernel(const Plan& p, const AggLayout& L, const KernelC
   o << "  }\n";
   o << "  if (mode_ == 2 || s_over_ == 0) break;\n";
   if (two) {
-    o << "  const bool again_ = s_room_ == GXA_G && s_many_ == 0;\n";
     o << "  __syncthreads();\n";
-    o << "  if (again_) { if (threadIdx.x == 0) { s_room_ = GXA_G2; s_rep_ = GXA_R2; } warps_init_(); }\n";
+    o << "  if (threadIdx.x == 0) gxa_next_split(&s_room_, &s_rep_, s_need_);\n";
+    o << "  __syncthreads();\n";
+    o << "  if (s_rep_ > 0) warps_init_();\n";
     o << "  else { mode_ = 2; table_init_(); }\n";
   } else {
     o << "  __syncthreads();\n";

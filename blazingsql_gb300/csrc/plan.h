@@ -128,10 +128,11 @@ std::string generate_agg_kernel(const Plan& plan, const AggLayout& L, const Kern
 // replica and warp) or, once more groups turn up, a hash table of `slots` groups.  Cell /
 // slot indices per accumulator; -1: it has none (a count has no sum, an input
 // that is never NULL no valid count).
-constexpr int kAggDict = 64;
+constexpr int kAggDict = 128;   // places of the dictionary: mostly empty, so that probes are short
+constexpr int kAggGroups = 64;  // groups with accumulators per warp, at most
 struct AggShared {
   int warp_groups = 0, replicas = 1, cells = 0, rows_cell = 0;
-  int warp_groups2 = 0, replicas2 = 1, cell_words = 0;  // a second split, for more groups; words of a cell per warp
+  int cell_words = 0;   // words of a cell per warp: groups x replicas, however they are split
   int slots = 0, accs = 0;
   bool packed = false;  // a group's keys are one word
   int dict_bytes = 0, dyn_bytes = 0;

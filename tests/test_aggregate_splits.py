@@ -1,6 +1,6 @@
-"""Group counts around the two splits of a warp's accumulators (few groups with
-many replicas, more groups with fewer), from the first rows on or only late, with
-keys that pack into one word and keys that do not."""
+"""Group counts around the splits of a warp's accumulators (few groups with many
+replicas, more groups with fewer), from the first rows on or only late, with keys
+that pack into one word and keys that do not."""
 import numpy as np
 import pytest
 
