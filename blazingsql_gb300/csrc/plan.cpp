@@ -245,19 +245,24 @@ int64_t ns_per_unit(int t) {
 class Gen {
  public:
   Gen(const Plan& p, const KernelConfig& c) : p_(p), cfg_(c) {
-    for (int r : p.conjuncts) prove_valid(r);
+    for (int r : p.conjuncts) {
+      const Node& n = p.nodes[r];
+      // IS NOT NULL proves its operand valid where it is true: as a conjunct
+      prove_valid(n.kind == Node::OP && n.op == OP_IS_NOT_NULL ? n.a : r);
+    }
   }
 
   // Columns that are valid in every row a conjunct keeps: a kept row's
   // conjunct is valid and true, and an operator that is NULL whenever an
-  // operand is makes its operands valid too.
+  // operand is makes its operands valid too.  The walk carries validity only,
+  // so it ends at operators that are valid whatever their operands are: under
+  // NOT or a comparison, IS NOT NULL($0) may be false in a kept row.
   void prove_valid(int id) {
     const Node& n = p_.nodes[id];
     if (n.kind == Node::COL) { proven_.insert(n.col); return; }
     if (n.kind != Node::OP) return;
     switch (n.op) {
-      case OP_IS_NOT_NULL: prove_valid(n.a); return;
-      case OP_OR: case OP_IS_NULL: case OP_IS_TRUE: case OP_IS_NOT_TRUE: case OP_IS_NOT_FALSE:
+      case OP_OR: case OP_IS_NULL: case OP_IS_NOT_NULL: case OP_IS_TRUE: case OP_IS_NOT_TRUE: case OP_IS_NOT_FALSE:
       case OP_IS_NOT_DISTINCT_FROM: case OP_MAGIC_IF_NOT: case OP_FIRST_NON_MAGIC: case OP_RAND: case OP_ROW_INDEX:
         return;
       default: break;
