@@ -3190,11 +3190,13 @@ std::string generate_agg_kernel(const Plan& p, const AggLayout& L, const KernelC
   // ---- merge into the global table
   o << "  if (mode_ == 1) {\n";
   o << "    const int ng_ = (int)min(s_ng_, s_room_); const int rep_ = s_rep_;\n";
-  o << "    if ((int)threadIdx.x < ng_) {\n";
-  o << "      const u32 i = d_at_[threadIdx.x];\n";
+  // a thread per group (a block of one warp has fewer threads than groups, so it goes round)
+  o << (cfg.warps * 32 >= kAggGroups ? "    if ((int)threadIdx.x < ng_) {\n      const int gi = (int)threadIdx.x;\n"
+                                     : "    for (int gi = (int)threadIdx.x; gi < ng_; gi += GX_WARPS * 32) {\n");
+  o << "      const u32 i = d_at_[gi];\n";
   o << "      u64 rows_ = 0ull;\n";  // none: its only round was left for the table
   o << "      for (int w = 0; w < GX_WARPS; w++)\n        for (int r = 0; r < rep_; r++)\n"
-       "          rows_ += s_warp_[" << sh.rows_cell << " * GXA_CS + w * GXA_GR + (int)threadIdx.x * rep_ + r];\n";
+       "          rows_ += s_warp_[" << sh.rows_cell << " * GXA_CS + w * GXA_GR + gi * rep_ + r];\n";
   o << "      u64 kv[GXA_NK]; kv[0] = 0ull;\n";
   if (sh.packed) {
     o << "      const u32 kn_ = gxa_unpack(d_ks_[i], kv);\n";
@@ -3202,7 +3204,7 @@ std::string generate_agg_kernel(const Plan& p, const AggLayout& L, const KernelC
     for (int j = 0; j < nk; j++) o << "      kv[" << j << "] = d_ks_[" << j << " * GXA_D + i];\n";
     o << "      const u32 kn_ = d_nm_[i];\n";
   }
-  o << "      d_gs_[threadIdx.x] = rows_ ? (u64)gxa_find_global(ga, kv, kn_, gxa_hash(kv, kn_)) : ~0ull;\n";
+  o << "      d_gs_[gi] = rows_ ? (u64)gxa_find_global(ga, kv, kn_, gxa_hash(kv, kn_)) : ~0ull;\n";
   o << "    }\n";
   o << "    __syncthreads();\n";
   // one warp per group and cell: lane w takes warp w's replicas, then a tree over lanes
