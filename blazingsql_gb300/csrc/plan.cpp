@@ -430,12 +430,14 @@ class Gen {
              // the condition has made the proven_ columns valid
   };
   mutable Masks masks_ = Masks::GLOBAL;
+  // a warp of more than 32 words has more of them than lanes: rows read their bits from the mask
+  bool lane_words() const { return cfg_.words <= 32; }
   bool masked(int c) const { return p_.nullable[c] && !(masks_ == Masks::KEPT && proven_.count(c)); }
   // validity of column c for the lane's row
   std::string col_valid(int c) const {
     const std::string cs = std::to_string(c);
     if (!masked(c)) return "inr";
-    switch (masks_) {
+    switch (lane_words() ? masks_ : Masks::GLOBAL) {
       case Masks::WORDS: return "(gx_wbit(mw_" + cs + ", k, lane) && inr)";
       case Masks::KEPT: return "(gx_wbit(mw_" + cs + ", kp_ >> 5, kp_ & 31u) && inr)";
       default: return "(inr && gx_valid(a.in_mask[" + cs + "], a.in_off[" + cs + "] + row))";
@@ -445,6 +447,7 @@ class Gen {
   // one word per lane (words w0 .. w0 + GX_V - 1)
   void emit_mask_words(std::ostringstream& o, const std::vector<int>& ids, const std::vector<int>& more,
                        const std::string& ind) const {
+    if (!lane_words()) return;
     std::set<int> cols(more.begin(), more.end());
     for (int id : ids)
       if (p_.nodes[id].kind == Node::COL) cols.insert(p_.nodes[id].col);
@@ -1316,7 +1319,9 @@ void emit_filter_writes_dense(std::ostringstream& o, const Gen& g, const Plan& p
     const OutSpec& os = p.outputs[j];
     if (os.kind == OutSpec::COPY ? g.masked(os.col) : !g.never_null(os.node)) slot[j] = nslots++;
   }
-  for (int sl = 0; sl < nslots; sl++) o << ind << "u32 vb" << sl << "_ = 0u;\n";
+  if (!g.lane_words()) o << ind << "const i64 cap_words = (a.capacity + 31) >> 5;\n";
+  else
+    for (int sl = 0; sl < nslots; sl++) o << ind << "u32 vb" << sl << "_ = 0u;\n";
   o << ind << "const u32 wmax_ = (u32)max((i64)0, min((i64)total_, a.capacity - (i64)pos));\n";
   o << ind << "for (u32 base_ = 0; base_ < total_; base_ += 32u) {\n";
   const std::string in2 = ind + "  ";
@@ -1335,16 +1340,19 @@ void emit_filter_writes_dense(std::ostringstream& o, const Gen& g, const Plan& p
   for (size_t j = 0; j < p.outputs.size(); j++) {
     const std::string v = emit_dense_store(o, g, p, j, in2);
     if (slot[j] < 0) continue;
-    o << in2 << "{ const u32 b_ = __ballot_sync(GX_FULL, " << v << " && act); if ((u32)lane == base_ >> 5) vb" << slot[j]
-      << "_ = b_; }\n";
+    o << in2 << "{ const u32 b_ = __ballot_sync(GX_FULL, " << v << " && act); ";
+    if (g.lane_words())
+      o << "if ((u32)lane == base_ >> 5) vb" << slot[j] << "_ = b_; }\n";
+    else  // more rounds than lanes: each round writes its own bits
+      o << "gx_put_bits(a.out_mask[" << j << "], (i64)pos + base_, min(32u, total_ - base_), lane == 0 ? b_ : 0u, cap_words); }\n";
   }
   o << ind << "}\n";
   o << ind << "__syncwarp();\n";  // the kept-row list and branch results are rewritten by the next tile
-  o << ind << "const i64 cap_words = (a.capacity + 31) >> 5;\n";
+  if (g.lane_words()) o << ind << "const i64 cap_words = (a.capacity + 31) >> 5;\n";
   for (size_t j : mo) {
-    if (slot[j] >= 0)
+    if (slot[j] >= 0 && g.lane_words())
       o << ind << "gx_put_bits(a.out_mask[" << j << "], (i64)pos, total_, vb" << slot[j] << "_, cap_words);\n";
-    else if (!listed)  // else the block writes its tile's (emit_tile_ones)
+    else if (slot[j] < 0 && !listed)  // else the block writes its tile's (emit_tile_ones)
       o << ind << "gx_put_ones(a.out_mask[" << j << "], (i64)pos, total_, cap_words);\n";
   }
   g.masks_ = was;
