@@ -23,6 +23,7 @@
 #include <algorithm>
 #include <array>
 #include <cstring>
+#include <deque>
 #include <map>
 #include <mutex>
 #include <type_traits>
@@ -1489,6 +1490,7 @@ struct Build {
   BuildArgs b{};
   XformArgs x{};
   unsigned nblocks = 0;
+  std::vector<std::string> lits;  // the literals' host bytes: their copy may still read them until the call waits
   uint64_t* sums = nullptr;  // the blocks' character totals, then their starts
   unsigned long long* total = nullptr;  // the character total, once the sizes are scanned
 };
@@ -1502,7 +1504,7 @@ static std::vector<unsigned long long*> g_slots;
 constexpr size_t kKeptSlots = 16;
 
 struct StringBuilds::State {
-  std::vector<Build> builds;
+  std::deque<Build> builds;  // (a build's literals stay where they are when one is added)
   unsigned long long* totals = nullptr;
 
   unsigned long long* slot(int i) {
@@ -1543,8 +1545,9 @@ int StringBuilds::size() const { return (int)st_->builds.size(); }
 // Allocates [mask | offsets | word starts | block sums | literals], uploads the
 // literals, and clears what the sizing launch does not write (the mask's
 // padding, the first offset of an empty column).
-static char* begin_build(Build& b, int64_t rows, const std::vector<std::string>& lits, std::vector<unsigned char*>* lit_dev,
+static char* begin_build(Build& b, int64_t rows, std::vector<std::string> lits, std::vector<unsigned char*>* lit_dev,
                          uint32_t** word_base, uint64_t** sums, cudaStream_t s) {
+  b.lits = std::move(lits);
   if (rows < 0 || rows > INT32_MAX) fail(GX_ERR_UNSUPPORTED, "string columns hold at most 2^31 - 1 rows");
   const int64_t words = mask_words_for(rows), used = (rows + 31) / 32;
   b.nblocks = (unsigned)((rows + kBuildRows - 1) / kBuildRows);
@@ -1552,7 +1555,7 @@ static char* begin_build(Build& b, int64_t rows, const std::vector<std::string>&
   const size_t mask_b = al((size_t)words * 4), offs_b = al((size_t)(rows + 1) * 4), word_b = al((size_t)(used + 1) * 4);
   const size_t sums_b = al((size_t)(b.nblocks + 1) * 8);
   size_t lit_b = 0;
-  for (const auto& l : lits) lit_b += al(l.size() + 1);
+  for (const auto& l : b.lits) lit_b += al(l.size() + 1);
   char* base = (char*)dev_alloc(mask_b + offs_b + word_b + sums_b + lit_b, s);
   b.out.type_id = STRING;
   b.out.null_mask = (uint32_t*)base;
@@ -1564,9 +1567,8 @@ static char* begin_build(Build& b, int64_t rows, const std::vector<std::string>&
   unsigned char* l = (unsigned char*)(base + mask_b + offs_b + word_b + sums_b);
   if (words > used) check_cuda(cudaMemsetAsync(base + used * 4, 0, (size_t)(words - used) * 4, s), "mask padding");
   if (rows == 0) check_cuda(cudaMemsetAsync(b.out.string_offsets, 0, 4, s), "empty offsets");
-  for (const auto& x : lits) {
+  for (const auto& x : b.lits) {
     lit_dev->push_back(l);
-    // (a copy from pageable memory returns once its bytes are staged)
     if (!x.empty()) check_cuda(cudaMemcpyAsync(l, x.data(), x.size(), cudaMemcpyHostToDevice, s), "string literal");
     l += al(x.size() + 1);
   }
@@ -2059,10 +2061,23 @@ std::vector<gx_column> run_string_prepass(std::vector<ColumnView>& cols, const s
     std::memcpy(&host[at], b->data(), b->size());
     at += slot(b->size());
   }
+  // A copy from pageable memory may return before it has read its source, so
+  // the patterns' host bytes stay until it is done: the scope's end waits for
+  // the copy (it leads the call's work, so it is over by then).
+  struct CopyDone {
+    cudaEvent_t event = nullptr;
+    ~CopyDone() {
+      if (!event) return;
+      cudaEventSynchronize(event);
+      cudaEventDestroy(event);
+    }
+  } copied;
   char* pdev = (char*)dev_alloc(host.size(), s);
   auto string_col = [&](int c) { return string_column(cols, c); };
   try {
+    check_cuda(cudaEventCreateWithFlags(&copied.event, cudaEventDisableTiming), "event");
     check_cuda(cudaMemcpyAsync(pdev, host.data(), host.size(), cudaMemcpyHostToDevice, s), "string patterns");
+    check_cuda(cudaEventRecord(copied.event, s), "event record");
     for (size_t i = 0; i < ops.size(); i++) {
       const StringOp& op = ops[i];
       gx_column out{};
@@ -2120,7 +2135,6 @@ std::vector<gx_column> run_string_prepass(std::vector<ColumnView>& cols, const s
     dev_free(pdev, s);
     throw;
   }
-  // (the patterns' copy returned once their pageable bytes were staged)
   dev_free(pdev, s);
   return made;
 }
