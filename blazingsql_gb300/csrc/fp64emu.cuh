@@ -467,15 +467,18 @@ GXE_FN gxe_u64 gxe_quot(gxe_u64 sign, int e, gxe_u64 A, gxe_u64 mb, gxe_u64 r) {
 
 // x / y for the operands no fast path takes: integers of more than 53
 // significant bits, divisors past a reciprocal table, subnormals, infinities,
-// NaNs, zero divisors.  The reciprocal and products of gxe_div inlined here cost the whole kernel 8 to 17 registers; this form keeps the
+// NaNs, zero divisors.  Same bits as gxe_div, whose reciprocal and products
+// inlined here cost the whole kernel 8 to 17 registers; this form keeps the
 // remainder, the divisor and the quotient alive.  Eleven quotient bits a step:
 // the digit is estimated from the leading 23 or 24 bits of both in binary32, off
 // by at most one, and the exact remainder corrects it.
 GXE_FN gxe_u64 gxe_div_rare(gxe_u64 a, gxe_u64 b) {
   const gxe_u64 sign = (a ^ b) & GXE_SIGN;
+  if (gxe_isnan_(a)) return GXE_QNAN | (a & (GXE_FRAC | GXE_SIGN));
+  if (gxe_isnan_(b)) return GXE_QNAN | (b & (GXE_FRAC | GXE_SIGN));
   a &= ~GXE_SIGN;
   b &= ~GXE_SIGN;
-  if (a > GXE_INF || b > GXE_INF || (a == b && (a == 0 || a == GXE_INF))) return GXE_QNAN;
+  if (a == b && (a == 0 || a == GXE_INF)) return GXE_QNAN | GXE_SIGN;
   if (a == GXE_INF || b == 0) return sign | GXE_INF;
   if (a == 0 || b == GXE_INF) return sign;
   int e = (int)(a >> 52) - (int)(b >> 52);
@@ -545,7 +548,7 @@ GXE_FN gxe_u64 gxe_div_k(gxe_u64 a, gxe_i64 k, const gxe_u64* rcp, int n) {
   // n < 2^20: the quotient's exponent stays normal for ea in [32, 2046]
   if (uk - 1ull >= (gxe_u64)n || (unsigned)(ea - 32) > 2014u) {
     const bool zero = (a << 1) == 0;
-    if (k == 0 && !gxe_isnan_(a)) return zero ? GXE_QNAN : (a & GXE_SIGN) | GXE_INF;
+    if (k == 0 && !gxe_isnan_(a)) return zero ? GXE_QNAN | GXE_SIGN : (a & GXE_SIGN) | GXE_INF;
     if (zero) return a ^ ((gxe_u64)k & GXE_SIGN);
     return gxe_div_rare(a, gxe_i2d(k));
   }
@@ -566,7 +569,7 @@ GXE_FN gxe_u64 gxe_divi_k(gxe_i64 x, gxe_i64 k, const gxe_u64* rcp, int n) {
   const int lx = gxe_clz(u);
   const gxe_u64 A = u << (lx & 63);
   if (uk - 1ull >= (gxe_u64)n || u == 0 || (A & 0x7FFull) != 0) {
-    if (k == 0) return u == 0 ? GXE_QNAN : ((gxe_u64)x & GXE_SIGN) | GXE_INF;
+    if (k == 0) return u == 0 ? GXE_QNAN | GXE_SIGN : ((gxe_u64)x & GXE_SIGN) | GXE_INF;
     if (u == 0) return (gxe_u64)k & GXE_SIGN;
     return gxe_div_rare(gxe_i2d(x), gxe_i2d(k));
   }
