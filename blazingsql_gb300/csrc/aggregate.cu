@@ -199,10 +199,14 @@ AggPlan::AggPlan(const std::vector<int>& schema, const std::vector<bool>& nullab
       out_types_.push_back(vt);
     }
   }
-  // one block per SM takes nearly all of its shared memory (227 KB less the
-  // kept-row lists and a margin)
+  // The registers leave room for 32 warps per SM, in one block or several, which
+  // share its 228 KB out by their warps (at most 208 KB in all), less a block's
+  // kept-row lists, the 1 KB that the hardware takes and the kernel's own words.
+  const int blocks = 32 / std::max(1, std::min(32, cfg_.warps));
+  const int taken = 1024 + cfg_.warps * cfg_.words * 64 + 512;
+  const int room = std::min(228 * 1024 / blocks - taken, 208 * 1024 / blocks);
   const int budget = std::getenv("GX_AGG_SMEM_KB") ? std::atoi(std::getenv("GX_AGG_SMEM_KB")) : 208;
-  layout_.smem_bytes = std::max(8, std::min(budget, 208)) * 1024;
+  layout_.smem_bytes = std::max(8 * 1024, std::min(std::max(8, std::min(budget, 208)) * 1024, room));
   const char* wc = std::getenv("GX_AGG_COMBINE");
   layout_.warp_combine = !(wc && *wc == '0');
 }

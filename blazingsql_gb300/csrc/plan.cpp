@@ -2687,7 +2687,7 @@ AggShared agg_shared(const Plan& p, const AggLayout& L, const KernelConfig& cfg)
     }
   }
   s.dict_bytes = (kAggDict * (8 * (nk + 1) + 12) + 15) / 16 * 16;
-  const int budget = L.smem_bytes - s.dict_bytes;
+  const int budget = std::max(L.smem_bytes - s.dict_bytes, 8 * 1024);  // small blocks keep a table of some size
   const int room = budget / (cfg.warps * s.cells * 8);  // words of a cell per warp
   s.replicas = std::max(1, std::min(16, room / 8));
   s.warp_groups = std::min(kAggGroups, room / s.replicas);

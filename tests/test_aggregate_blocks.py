@@ -1,7 +1,8 @@
 """The aggregation kernel in blocks of other sizes than its own 32 warps, as
 GX_WARPS / GX_WORDS ask for: group counts on both sides of a one-warp block's
-32 threads and of the 64 groups that have accumulators per warp, with keys that
-pack into one word and keys that do not."""
+32 threads and of the 64 groups that have accumulators per warp, blocks whose
+kept-row lists take much of the shared memory, with keys that pack into one word
+and keys that do not."""
 import numpy as np
 import pytest
 
@@ -21,7 +22,7 @@ def _table(n, groups):
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("groups", [1, 31, 32, 33, 63, 64, 65, 3000])
-@pytest.mark.parametrize("shape", [(1, 4), (1, 8), (2, 4), (4, 8), (0, 0)], ids=str)
+@pytest.mark.parametrize("shape", [(1, 4), (1, 8), (2, 4), (4, 8), (16, 8), (32, 16), (16, 32), (0, 0)], ids=str)
 def test_group_counts_by_block(shape, groups, monkeypatch):
     if shape[0]:
         monkeypatch.setenv("GX_WARPS", str(shape[0]))
