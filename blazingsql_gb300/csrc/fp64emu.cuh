@@ -465,13 +465,12 @@ GXE_FN gxe_u64 gxe_quot(gxe_u64 sign, int e, gxe_u64 A, gxe_u64 mb, gxe_u64 r) {
   return sign | (((gxe_u64)(unsigned)(e - 1 - s) << 52) + m + up);
 }
 
-// x / y for the operands no fast path takes: integers of more than 53
-// significant bits, divisors past a reciprocal table, subnormals, infinities,
-// NaNs, zero divisors.  Same bits as gxe_div, whose reciprocal and products
-// inlined here cost the whole kernel 8 to 17 registers; this form keeps the
-// remainder, the divisor and the quotient alive.  Eleven quotient bits a step:
-// the digit is estimated from the leading 23 or 24 bits of both in binary32, off
-// by at most one, and the exact remainder corrects it.
+// x / y for the operands no fast path takes: subnormals, infinities, NaNs, zero
+// divisors, quotients outside the normal range.  Same bits as gxe_div, whose
+// reciprocal and products inlined here cost the whole kernel 8 to 17 registers;
+// this form keeps the remainder, the divisor and the quotient alive.  Eleven
+// quotient bits a step: the digit is estimated from the leading 23 or 24 bits of
+// both in binary32, off by at most one, and the exact remainder corrects it.
 GXE_FN gxe_u64 gxe_div_rare(gxe_u64 a, gxe_u64 b) {
   const gxe_u64 sign = (a ^ b) & GXE_SIGN;
   if (gxe_isnan_(a)) return GXE_QNAN | (a & (GXE_FRAC | GXE_SIGN));
@@ -525,61 +524,103 @@ GXE_FN gxe_u64 gxe_div_lit(gxe_u64 a, gxe_u64 b, gxe_u64 r) {
   return gxe_quot((a ^ b) & GXE_SIGN, ea - eb + 1023, A, (b & GXE_FRAC) | GXE_HIDDEN, r);
 }
 
+// A 64-bit integer with its top bit set, rounded to its leading 53 bits as the
+// conversion to binary64 rounds it (nearest, ties to even); true on a carry,
+// which leaves 2^63 and one more in the exponent.
+GXE_FN bool gxe_round53(gxe_u64* A) {
+  if ((*A & 0x7FFull) == 0) return false;
+  const gxe_u64 t = *A + 0x3FFull + ((*A >> 11) & 1ull);
+  const bool carry = t < *A;
+  *A = carry ? 1ull << 63 : t & ~0x7FFull;
+  return carry;
+}
+
 // (double)x / b for a literal b and an integer x: as gxe_div_lit, without the
-// conversion (an x of more than 53 significant bits converts first)
+// conversion
 GXE_FN gxe_u64 gxe_divi_lit(gxe_i64 x, gxe_u64 b, gxe_u64 r) {
   const int eb = (int)((b >> 52) & 0x7FF);
   const gxe_u64 u = x < 0 ? 0ull - (gxe_u64)x : (gxe_u64)x;
   const gxe_u64 sign = ((gxe_u64)x ^ b) & GXE_SIGN;
   const int lz = gxe_clz(u);
-  const gxe_u64 A = u << (lz & 63);
-  const int e = 1023 + 63 - lz - eb + 1023;
+  gxe_u64 A = u << (lz & 63);
+  int e = 1023 + 63 - lz - eb + 1023;
   if (u == 0) return sign;
-  if ((A & 0x7FFull) != 0 || (unsigned)(e - 2) > 2044u) return gxe_div_rare(gxe_i2d(x), b);
+  if (gxe_round53(&A)) e++;
+  if ((unsigned)(e - 2) > 2044u) return gxe_div_rare(gxe_i2d(x), b);
   return gxe_quot(sign, e, A, (b & GXE_FRAC) | GXE_HIDDEN, r);
 }
 
-// x / k for an integer k: rcp[i] = gxe_recip_floor(significand of i + 1),
-// used for 1 <= |k| <= n.  Zeros of either side are answered here: a filter's
-// idle lanes divide 0 by 0, and must not draw their warp into the rare path.
+// A / (mb 2^11) as gxe_quot, without a reciprocal: a first quotient bit, then
+// three digits of 20 bits, each estimated in binary32 from the leading 24 bits of
+// the remainder and the divisor, off by at most one, and corrected by the exact
+// remainder.  It keeps few values alive: gxe_recip_fixed in its place costs the
+// order-line plan 10 registers of 68.
+GXE_FN gxe_u64 gxe_quot_steps(gxe_u64 sign, int e, gxe_u64 A, gxe_u64 mb) {
+  gxe_u64 m = A >> 11;
+  if (m < mb) { m <<= 1; e--; }
+  m -= mb;
+  gxe_u64 q = 1;
+  const float inv = 1048576.0f * gxe_rcp_approx((float)(unsigned)(mb >> 29));
+#if GXE_ON_DEVICE
+#pragma unroll 1
+#endif
+  for (int i = 0; i < 3; i++) {  // m < mb < 2^53
+    unsigned digit = (unsigned)((float)(unsigned)(m >> 29) * inv);
+    m = (m << 20) - (gxe_u64)digit * mb;  // in [-mb, 2 mb)
+    if ((gxe_i64)m < 0) { digit--; m += mb; }
+    else if (m >= mb) { digit++; m -= mb; }
+    q = (q << 20) + digit;
+  }
+  return sign | (((gxe_u64)(unsigned)(e - 1) << 52) + (q >> 8) + ((q >> 7) & 1ull));
+}
+
+// A / (the double of |k| = uk, times 2^11) for an integer divisor, e the biased
+// exponent of the quotient by one: the table's reciprocal for uk <= n, else by
+// steps.  Call us, 2^25 rows, doubles by integers up to 10^6 / integers by them /
+// 62-bit integers by 7.0: 433 / 437 / 287 with gxe_div for what no table serves and
+// the FMA unit for the rest, 516 / 492 / 381 with gxe_div_rare, 320 / 340 / 164 now.
+GXE_FN gxe_u64 gxe_quot_k(gxe_u64 sign, int e, gxe_u64 A, gxe_u64 uk, const gxe_u64* rcp, int n) {
+  const int lz = gxe_clz(uk);
+  gxe_u64 m = uk << (lz & 63);
+  e += lz - 63;
+  if (uk - 1ull < (gxe_u64)n) {
+#if GXE_ON_DEVICE
+    const gxe_u64 r = __ldg(rcp + (uk - 1ull));
+#else
+    const gxe_u64 r = rcp[uk - 1ull];
+#endif
+    return gxe_quot(sign, e, A, m >> 11, r);
+  }
+  if (gxe_round53(&m)) e--;
+  return gxe_quot_steps(sign, e, A, m >> 11);
+}
+
+// x / k for an integer k: rcp[i] = gxe_recip_floor(significand of i + 1), for
+// 1 <= |k| <= n.  Zeros of either side are answered here: a filter's idle lanes
+// divide 0 by 0, and must not draw their warp into the rare path.
 GXE_FN gxe_u64 gxe_div_k(gxe_u64 a, gxe_i64 k, const gxe_u64* rcp, int n) {
   const gxe_u64 uk = k < 0 ? 0ull - (gxe_u64)k : (gxe_u64)k;
   const int ea = (int)((a >> 52) & 0x7FF);
-  // n < 2^20: the quotient's exponent stays normal for ea in [32, 2046]
-  if (uk - 1ull >= (gxe_u64)n || (unsigned)(ea - 32) > 2014u) {
+  // |k| <= 2^63: the quotient's exponent stays normal for ea in [66, 2046]
+  if (k == 0 || (unsigned)(ea - 66) > 1980u) {
     const bool zero = (a << 1) == 0;
     if (k == 0 && !gxe_isnan_(a)) return zero ? GXE_QNAN | GXE_SIGN : (a & GXE_SIGN) | GXE_INF;
     if (zero) return a ^ ((gxe_u64)k & GXE_SIGN);
     return gxe_div_rare(a, gxe_i2d(k));
   }
-  const int lz = gxe_clz(uk);
-#if GXE_ON_DEVICE
-  const gxe_u64 r = __ldg(rcp + (uk - 1ull));
-#else
-  const gxe_u64 r = rcp[uk - 1ull];
-#endif
-  const gxe_u64 A = ((a & GXE_FRAC) | GXE_HIDDEN) << 11;
-  return gxe_quot((a ^ (gxe_u64)k) & GXE_SIGN, ea - (63 - lz), A, uk << (lz - 11), r);
+  return gxe_quot_k((a ^ (gxe_u64)k) & GXE_SIGN, ea, ((a & GXE_FRAC) | GXE_HIDDEN) << 11, uk, rcp, n);
 }
 
 // (double)x / (double)k for integers: as gxe_div_k, without the conversions
 GXE_FN gxe_u64 gxe_divi_k(gxe_i64 x, gxe_i64 k, const gxe_u64* rcp, int n) {
   const gxe_u64 uk = k < 0 ? 0ull - (gxe_u64)k : (gxe_u64)k;
   const gxe_u64 u = x < 0 ? 0ull - (gxe_u64)x : (gxe_u64)x;
-  const int lx = gxe_clz(u);
-  const gxe_u64 A = u << (lx & 63);
-  if (uk - 1ull >= (gxe_u64)n || u == 0 || (A & 0x7FFull) != 0) {
-    if (k == 0) return u == 0 ? GXE_QNAN | GXE_SIGN : ((gxe_u64)x & GXE_SIGN) | GXE_INF;
-    if (u == 0) return (gxe_u64)k & GXE_SIGN;
-    return gxe_div_rare(gxe_i2d(x), gxe_i2d(k));
-  }
-  const int lz = gxe_clz(uk);
-#if GXE_ON_DEVICE
-  const gxe_u64 r = __ldg(rcp + (uk - 1ull));
-#else
-  const gxe_u64 r = rcp[uk - 1ull];
-#endif
-  return gxe_quot(((gxe_u64)x ^ (gxe_u64)k) & GXE_SIGN, 1023 + lz - lx, A, uk << (lz - 11), r);
+  if (k == 0) return u == 0 ? GXE_QNAN | GXE_SIGN : ((gxe_u64)x & GXE_SIGN) | GXE_INF;
+  if (u == 0) return (gxe_u64)k & GXE_SIGN;
+  int lx = gxe_clz(u);
+  gxe_u64 A = u << lx;
+  if (gxe_round53(&A)) lx--;
+  return gxe_quot_k(((gxe_u64)x ^ (gxe_u64)k) & GXE_SIGN, 1023 + 63 - lx, A, uk, rcp, n);
 }
 
 // (double)v of an integer known to fit 32 bits: one shift instead of the
