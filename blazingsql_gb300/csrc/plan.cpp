@@ -1429,6 +1429,41 @@ void emit_filter_writes(std::ostringstream& o, const Gen& g, const Plan& p, cons
   }
 }
 
+// The tile pipeline's kept-row lists, in shared memory: one of each tile in
+// flight, made with the tile's predicate.  A block whose rows (or expensive CASE
+// branches) leave no room for two of them in the 227 KB that it may have keeps the
+// next tile's keep masks, a 16th of the size, and lists them when it writes.
+struct KeptLists {
+  bool two = true;
+  KeptLists(const Gen& g) {
+    const size_t rows = (size_t)g.cfg_.warps * g.cfg_.words * 32, branches = g.lazy_branches(g.output_roots()).size();
+    const size_t others = (size_t)g.cfg_.warps * (24 + 4 * g.cfg_.words) + 256;  // counts, offsets, the tile's words
+    two = rows * (4 + (branches ? 2 : 0) + 9 * branches) + others <= 227 * 1024;
+  }
+  void decl(std::ostringstream& o) const {
+    o << "  __shared__ unsigned short s_kept_[" << (two ? 2 : 1) << "][GX_WARPS][GX_V * 32];\n";
+    if (!two) o << "  __shared__ u32 s_bal_[2][GX_WARPS][GX_V];\n";
+  }
+  // keeps the warp's rows of bal[] for tile slot `buf`, counting them in `cnt`
+  void keep(std::ostringstream& o, const std::string& buf, const std::string& cnt, const std::string& ind) const {
+    if (two) return emit_kept_list(o, "bal", "s_kept_[" + buf + "][warp]", cnt, ind);
+    o << ind << "#pragma unroll\n" << ind << "for (int kk = 0; kk < GX_V; kk++) {\n";
+    o << ind << "  if (lane == 0) s_bal_[" << buf << "][warp][kk] = bal[kk];\n" << ind << "  " << cnt
+      << " += __popc(bal[kk]);\n" << ind << "}\n";
+    o << ind << "__syncwarp();\n";
+  }
+  // kl_ and total_ of the tile in slot par
+  void list(std::ostringstream& o, const std::string& ind) const {
+    if (!two) {
+      o << ind << "u32 listed_ = 0u; u32 wb_[GX_V];\n";
+      o << ind << "#pragma unroll\n" << ind << "for (int kk = 0; kk < GX_V; kk++) wb_[kk] = s_bal_[par][warp][kk];\n";
+      emit_kept_list(o, "wb_", "s_kept_[0][warp]", "listed_", ind);
+      o << ind << "__syncwarp();\n";
+    }
+    o << ind << "const unsigned short* const kl_ = s_kept_[" << (two ? "par" : "0") << "][warp]; const u32 total_ = wcnt;\n";
+  }
+};
+
 // Fused single-pass filter (dense projections) as a two-stage tile pipeline:
 // a block evaluates tile t+1's predicate before it resolves tile t's output
 // offset by look-back, so the look-back of t waits on tiles that had a whole
@@ -1463,7 +1498,8 @@ void emit_fused_pipelined(std::ostringstream& o, const Gen& g, const Plan& p, co
   o << "  __shared__ u32 s_cnt[2][GX_WARPS];\n";
   o << "  __shared__ u64 s_off[2][GX_WARPS];\n";
   o << "  __shared__ u64 s_base, s_total;\n";
-  o << "  __shared__ unsigned short s_kept_[2][GX_WARPS][GX_V * 32];\n";
+  const KeptLists kept(g);
+  kept.decl(o);
   o << "  const i64 ntiles = (nwords + GX_TILE_WORDS - 1) / GX_TILE_WORDS;\n";
   o << "  if (threadIdx.x == 0) s_claim = atomicAdd(a.tile_counter, 1ull);\n";
   o << "  __syncthreads();\n";
@@ -1481,7 +1517,7 @@ void emit_fused_pipelined(std::ostringstream& o, const Gen& g, const Plan& p, co
     count_conjuncts(ind);
     o << ind << "u32 bal[GX_V];\n";
     o << ind << "#pragma unroll\n" << ind << "for (int k = 0; k < GX_V; k++) bal[k] = __ballot_sync(GX_FULL, alive[k]);\n";
-    emit_kept_list(o, "bal", "s_kept_[" + buf + "][warp]", cnt, ind);
+    kept.keep(o, buf, cnt, ind);
     o << ind << "if (lane == 0) s_cnt[" << buf << "][warp] = " << cnt << ";\n";
   };
   predicate("0", "wcnt", "    ");
@@ -1517,7 +1553,7 @@ void emit_fused_pipelined(std::ostringstream& o, const Gen& g, const Plan& p, co
   o << "    if (wcnt != 0u) {\n";
   o << "      u64 pos = base_t + s_off[par][warp];\n";
   o << "      const i64 w0 = tile * GX_TILE_WORDS + (i64)warp * GX_V;\n";
-  o << "      const unsigned short* const kl_ = s_kept_[par][warp]; const u32 total_ = wcnt;\n";
+  kept.list(o, "      ");
   emit_filter_writes_dense(o, g, p, "      ", true);
   o << "    }\n";
   o << "    if (next >= ntiles) break;\n";
@@ -1983,7 +2019,8 @@ void emit_fused_batched(std::ostringstream& o, const Gen& g, const Plan& p, cons
   o << "  __shared__ u32 s_cnt[2][GX_WARPS];\n";
   o << "  __shared__ u64 s_off[2][GX_WARPS];\n";
   o << "  __shared__ u64 s_base, s_total;\n";
-  o << "  __shared__ unsigned short s_kept_[2][GX_WARPS][GX_V * 32];\n";
+  const KeptLists kept(g);
+  kept.decl(o);
   // the batch of global tile gt, at or after batch b
   auto find = [&](const std::string& b, const std::string& gt, const std::string& ind) {
     if (streaming) o << ind << "while (" << b << " + 1 < nbatch && tile_base[" << b << " + 1] <= " << gt << ") " << b << "++;\n";
@@ -2017,7 +2054,7 @@ void emit_fused_batched(std::ostringstream& o, const Gen& g, const Plan& p, cons
     g.emit_predicate(o, ind);
     o << ind << "u32 bal[GX_V];\n";
     o << ind << "#pragma unroll\n" << ind << "for (int k = 0; k < GX_V; k++) bal[k] = __ballot_sync(GX_FULL, alive[k]);\n";
-    emit_kept_list(o, "bal", "s_kept_[" + buf + "][warp]", cnt, ind);
+    kept.keep(o, buf, cnt, ind);
     o << ind << "if (lane == 0) s_cnt[" << buf << "][warp] = " << cnt << ";\n";
   };
   o << "  {\n";
@@ -2071,7 +2108,7 @@ void emit_fused_batched(std::ostringstream& o, const Gen& g, const Plan& p, cons
   o << "      const GxArgs& a = GX_BATCH(pb);\n";
   o << "      u64 pos = base_t + s_off[par][warp];\n";
   o << "      const i64 w0 = tile * GX_TILE_WORDS + (i64)warp * GX_V;\n";
-  o << "      const unsigned short* const kl_ = s_kept_[par][warp]; const u32 total_ = wcnt;\n";
+  kept.list(o, "      ");
   emit_filter_writes_dense(o, g, p, "      ", true);
   o << "    }\n";
   o << "    if (next < 0) break;\n";
