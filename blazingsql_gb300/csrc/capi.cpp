@@ -907,6 +907,7 @@ static std::string debug_source(const gx_plan* plan, int kind, const uint8_t* ha
     cfg.runtime_order = kind == 4 || kind == 7;
     cfg.staged = kind == 7;
     if (kind == 4) {  // as the learner builds it
+      if (copies_only(p) && cfg.tune_shape) cfg.warps = 8;
       const char* st = std::getenv("GX_STREAM");
       cfg.stream_slots = st && *st ? std::atoi(st) : 0;
     }

@@ -618,18 +618,11 @@ static std::shared_ptr<CompiledPlan> variant(const CompiledPlan& base, int mode,
     // so on request only (GX_STREAM=<slots>)
     const char* st = std::getenv("GX_STREAM");
     c.stream_slots = st && *st ? std::atoi(st) : 0;
-    // The ordered kernel waits on one load per conjunct and word, so resident
-    // warps are what hides it: with outputs that are column copies, few values
-    // are live and 32 registers (64 warps per SM) suffice.  Eight batches of 2^23
-    // rows, two copied outputs: 0.63 ms, 0.66 at 40 registers, 0.72 at 48, 0.83
-    // uncapped (72).  Computed outputs would spill, so they stay uncapped.
-    bool copies = true;
-    for (const auto& os : base.plan().outputs) copies = copies && os.kind == OutSpec::COPY;
-    if (copies && c.max_regs == 0) c.max_regs = 32;
-    // Blocks of 8 warps start half as many tiles' look-backs as blocks of 4: the
-    // same eight batches 0.55 ms instead of 0.59 (16 warps 0.54, but a small
-    // batch then fills few blocks).  A shape that the caller chose stays.
-    if (copies && base.config().tune_shape) c.warps = 8;
+    // With column copies as outputs, blocks of 8 warps start half as many tiles'
+    // look-backs as blocks of 4: eight batches of 2^23 rows, two copied outputs,
+    // 0.55 ms instead of 0.59 (16 warps 0.54, but a small batch then fills few
+    // blocks).  A shape that the caller chose stays.
+    if (copies_only(base.plan()) && base.config().tune_shape) c.warps = 8;
   }
   return std::make_shared<CompiledPlan>(base.plan(), c, mode);
 }

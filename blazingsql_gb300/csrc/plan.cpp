@@ -2480,8 +2480,41 @@ static bool project_fits_cap(const Plan& p, const KernelConfig& cfg) {
   return fits && regs <= kProjectRegs / 2;
 }
 
+bool copies_only(const Plan& p) {
+  for (const auto& o : p.outputs)
+    if (o.kind != OutSpec::COPY) return false;
+  return true;
+}
+
+// The learner's ordered kernel waits on one load per conjunct and word, so
+// resident warps are what hides it: with outputs that are column copies, few
+// values are live, and 32 registers (64 warps per SM) suffice for conjuncts that
+// compare and add.  Validity and divisions keep more alive, and 48 registers then
+// spill less than the lost warps cost; a transcendental function's own state spills
+// at either, and 40 keep more warps.  Queues of eight batches of 2^22 rows, us
+// at 32 / 40 / 48 registers / uncapped: the skewed-range conjuncts 481 / 521 / 537
+// / 888, over nullable columns 641 / 553 / 543 / 840; sums 728 / 837 / 810 / 1374
+// and 976 / 881 / 851 / 1803; divisions 1782 / 1620 / 1527 / 1737 and 1949 / 1876 /
+// 1753 / 3177; LN and EXP 3771 / 3577 / 3757 / 3662 and 3832 / 3610 / 3722 / 3781.
+static int ordered_regs(const Plan& p) {
+  bool nulls = false;
+  int most = 0;  // the dearest operator's cost
+  std::function<void(int)> go = [&](int id) {
+    if (id < 0) return;
+    const Node& n = p.nodes[id];
+    if (n.kind == Node::COL) nulls = nulls || p.nullable[n.col];
+    if (n.kind != Node::OP) return;
+    most = std::max(most, Gen::op_cost(n.op));
+    go(n.a);
+    go(n.b);
+  };
+  for (int c : p.conjuncts) go(c);
+  return most >= 64 ? 40 : most >= 16 || nulls ? 48 : 32;
+}
+
 std::string generate_kernel(const Plan& p, KernelKind kind, const KernelConfig& cfg_in, const std::string& name) {
   KernelConfig cfg = cfg_in;
+  if (cfg.runtime_order && cfg.max_regs == 0 && copies_only(p)) cfg.max_regs = ordered_regs(p);
   if (cfg.native_f64_ops < 0) cfg.native_f64_ops = auto_native_f64_ops();
   if (kind == KernelKind::PROJECT && cfg.max_regs == 0 && project_fits_cap(p, cfg)) cfg.max_regs = kProjectRegs;
   Gen g(p, cfg);

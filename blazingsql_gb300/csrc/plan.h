@@ -109,6 +109,9 @@ Plan build_plan(const std::vector<int>& schema, const std::vector<bool>& nullabl
 // NODE output computed in the kernel -- the aggregation kernel reads values
 // from nodes only; a bare literal is rejected there)
 
+// Every output is a column copied by kept row.
+bool copies_only(const Plan& plan);
+
 // Fused filter + group-by aggregation (gx_filter_aggregate): the plan's
 // outputs are the key columns then the non-empty aggregation inputs, all NODE
 // outputs.  The kernel keeps a block's groups in shared memory and merges them
