@@ -655,6 +655,11 @@ __device__ __forceinline__ u32 gx_lds_acquire(const u32* p) {
   asm volatile("ld.acquire.cta.shared::cta.u32 %0, [%1];" : "=r"(v) : "r"(gx_saddr(p)) : "memory");
   return v;
 }
+__device__ __forceinline__ u32 gx_ldg_acquire(const u32* p) {
+  u32 v;
+  asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
 // 64-bit add in shared memory as two 32-bit atomics, the carry with the second
 __device__ __forceinline__ void gx_sadd64(u64* p, u64 x) {
   const u32 lo = (u32)x, old = atomicAdd((u32*)p, lo);
