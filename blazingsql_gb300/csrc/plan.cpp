@@ -388,8 +388,13 @@ class Gen {
     bool any = false;
     for (size_t i = 0; i < p_.nodes.size() && !any; i++) any = small_div((int)i);
     if (!any) return;
-    static const std::string tables[2] = {rcp_table(false), rcp_table(true)};
-    o << tables[emu_op(kNativeIntDiv) ? 1 : 0];
+    if (emu_op(kNativeIntDiv)) {
+      static const std::string fixed = rcp_table(true);
+      o << fixed;
+    } else {
+      static const std::string binary64 = rcp_table(false);
+      o << binary64;
+    }
   }
   static std::string rcp_table(bool fixed) {
     std::ostringstream o;
