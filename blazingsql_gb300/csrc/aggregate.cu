@@ -126,6 +126,13 @@ bool key_type_ok(int t) {
   return (t >= INT8 && t <= UINT64) || t == BOOL8 || (t >= TIMESTAMP_DAYS && t <= DURATION_NANOSECONDS);
 }
 
+// Plans of this many accumulators take blocks of 16 warps with 128 registers a
+// thread: at 32 warps and 64 registers 24 sums, MIN and MAX of nullable columns
+// spill 1138 bytes.  Call us at 32 / 16 warps, 2^24 rows: these by 6 groups 1994 /
+// 1587, by 2557 groups 6753 / 4321; 24 sums of products 1757 / 1741 and 4332 / 2974.
+// 16 general divisions (16 accumulators) stay at 32 warps: 4334 / 5457.
+constexpr size_t kWideAccumulators = 20;
+
 uint64_t next_pow2(uint64_t x) {
   uint64_t p = 1;
   while (p < x) p <<= 1;
@@ -199,14 +206,36 @@ AggPlan::AggPlan(const std::vector<int>& schema, const std::vector<bool>& nullab
       out_types_.push_back(vt);
     }
   }
+  // How much of the SM's 256 KB the tables take: what they leave is L1, which the
+  // rounds' loads and spilled values need.  186 KB and the kernel's own words are
+  // the step below the whole SM; keys of at most 16 bits have few groups, whose
+  // replicas are worth the rest, and small calls pay for clearing and merging a
+  // table.  Nine aggregations, call us at 208 / 176 / 144 / 104 KB, 2^24 rows: 6
+  // groups by a 64-bit key 468 / 417 / 425 / 427, 2557 groups 620 / 593 / 605 / 706,
+  // 10,000 groups 1766 / 1042 / 1054 / 1101; 16 divisions by one byte 4328 / 4859 /
+  // 4845 / 4765; 300,000 rows by 2557 groups 189, with 64 KB 162.
+  int most = 208;
+  if (cfg_.tune_shape) {
+    int key_bits = 0;
+    for (int t : key_types_) key_bits += 8 * type_size(t);
+    if (key_bits > 16) {
+      most = 186;
+      // wider keys have more groups: the first split has room for 20 of them (18
+      // groups by a 64-bit key, 2^24 / 2^20 / 10^5 rows: 468 / 152 / 124 us with 8,
+      // 441 / 134 / 120 with 20; 6 groups 421 / 131 / 110 and 436 / 135 / 114)
+      layout_.first_groups = 20;
+    }
+    if (cfg_.warps < 32) most = 64;
+    if (layout_.kinds.size() >= kWideAccumulators) cfg_.warps = 16;
+  }
+  if (const char* kb = std::getenv("GX_AGG_SMEM_KB")) most = std::max(8, std::min(std::atoi(kb), 208));
   // The registers leave room for 32 warps per SM, in one block or several, which
   // share its 228 KB out by their warps (at most 208 KB in all), less a block's
   // kept-row lists, the 1 KB that the hardware takes and the kernel's own words.
   const int blocks = 32 / std::max(1, std::min(32, cfg_.warps));
   const int taken = 1024 + cfg_.warps * cfg_.words * 64 + 512;
   const int room = std::min(228 * 1024 / blocks - taken, 208 * 1024 / blocks);
-  const int budget = std::getenv("GX_AGG_SMEM_KB") ? std::atoi(std::getenv("GX_AGG_SMEM_KB")) : 208;
-  layout_.smem_bytes = std::max(8 * 1024, std::min(std::max(8, std::min(budget, 208)) * 1024, room));
+  layout_.smem_bytes = std::max(8 * 1024, std::min(most * 1024, room));
   const char* wc = std::getenv("GX_AGG_COMBINE");
   layout_.warp_combine = !(wc && *wc == '0');
 }

@@ -589,9 +589,12 @@ int gx_filter_project(const gx_column_view* columns, int num_columns, const char
   });
 }
 
+constexpr int64_t kAggSmallRows = int64_t(1) << 19;
+
 static std::shared_ptr<AggPlan> agg_plan_for(const std::vector<int>& schema, const std::vector<bool>& nullable,
                                              const char* condition, const int* group_columns, int nk,
-                                             const char* const* agg_inputs, const int* agg_kinds, int na) {
+                                             const char* const* agg_inputs, const int* agg_kinds, int na,
+                                             int64_t rows) {
   if (nk < 0 || na <= 0 || (nk > 0 && !group_columns) || !agg_inputs || !agg_kinds)
     fail(GX_ERR_INVALID, "bad aggregation arguments");
   std::string cond = condition ? std::string(condition) : std::string();
@@ -609,9 +612,11 @@ static std::shared_ptr<AggPlan> agg_plan_for(const std::vector<int>& schema, con
     // ticket is 128 rows.  Kernel us, nine aggregations by two flags (2^26 rows) /
     // four by ship date (2^24): 32 x 4 1298 / 545, 32 x 8 1297 / 553, 28 x 4
     // 1378 / 645; with combining trees for both, 24 x 8 1782 / 700, 16 x 8 2257 /
-    // 934.
-    cfg.warps = 32;
-    cfg.words = 4;
+    // 934.  Small calls leave most warps without a ticket: call us at 32 x 4 / 16 x
+    // 2, 24 nullable aggregations 218 / 172 at 10^5 rows, 240 / 187 at 2^18; 16
+    // divisions 269 / 184 and 283 / 227; at 2^20 445 / 473.
+    cfg.warps = rows < kAggSmallRows ? 16 : 32;
+    cfg.words = rows < kAggSmallRows ? 2 : 4;
   }
   std::string key;
   for (size_t i = 0; i < schema.size(); i++) key += std::to_string(schema[i]) + (nullable[i] ? "n," : "-,");
@@ -647,7 +652,7 @@ int gx_filter_aggregate(const gx_column_view* columns, int num_columns, const ch
     std::vector<bool> nullable;
     for (const auto& c : cols) nullable.push_back(c.mask != nullptr);
     auto ap = agg_plan_for(schema_of(cols), nullable, condition, group_columns, num_group_columns, agg_inputs,
-                           agg_kinds, num_aggs);
+                           agg_kinds, num_aggs, cols.empty() ? 0 : cols[0].size);
     for (int i = 0; i < ap->num_outputs(); i++) out[i] = gx_column{};
     ap->execute(cols, out, out_groups, (cudaStream_t)stream);
   });
@@ -663,7 +668,7 @@ int gx_debug_aggregate_check(const int32_t* column_types, const uint8_t* column_
     std::vector<bool> nullable;
     for (int i = 0; i < num_columns; i++) nullable.push_back(column_has_mask ? column_has_mask[i] != 0 : true);
     auto ap = agg_plan_for(schema, nullable, condition, group_columns, num_group_columns, agg_inputs, agg_kinds,
-                           num_aggs);
+                           num_aggs, kAggSmallRows);
     const KernelResources r = jit_resources(ap->kernel_source(nullable), "gx_filter_aggregate");
     if (registers) *registers = r.registers;
     if (spill_bytes) *spill_bytes = r.spill_bytes;

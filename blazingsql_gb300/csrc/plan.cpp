@@ -2771,7 +2771,7 @@ AggShared agg_shared(const Plan& p, const AggLayout& L, const KernelConfig& cfg)
   s.dict_bytes = (kAggDict * (8 * (nk + 1) + 12) + 15) / 16 * 16;
   const int budget = std::max(L.smem_bytes - s.dict_bytes, 8 * 1024);  // small blocks keep a table of some size
   const int room = budget / (cfg.warps * s.cells * 8);  // words of a cell per warp
-  s.replicas = std::max(1, std::min(16, room / 8));
+  s.replicas = std::max(1, std::min(16, room / L.first_groups));
   s.warp_groups = std::min(kAggGroups, room / s.replicas);
   s.cell_words = std::min(room, s.replicas * kAggGroups);
   const int slot_bytes = 8 * ((s.packed ? 1 : nk) + s.accs) + 4 * ((s.packed ? 1 : 3) + cnts);

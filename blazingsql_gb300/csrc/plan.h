@@ -121,6 +121,7 @@ struct AggLayout {
   std::vector<int> kinds;       // gx_agg_kind per aggregation
   std::vector<int> in_nodes;    // input node per aggregation (-1: COUNT(*))
   int smem_bytes = 0;           // dynamic shared memory a block may take
+  int first_groups = 8;         // groups that the accumulators' first split has room for
   // the lanes of one group combine their inputs over a warp tree before one
   // lane applies them (true), or every lane applies its own row (false)
   bool warp_combine = true;
