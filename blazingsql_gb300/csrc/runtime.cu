@@ -487,12 +487,11 @@ static const char* kind_name(KernelKind k) {
 
 // Candidate block shapes (warps x words, register cap) of a tuned single-pass
 // filter: the first is used until the others have been measured.  Measured on
-// GB300 (kernel us; light C1 plan 2^24 rows / deep C2 2^26 / order-line C5 2^27 /
-// process_filter of six columns 2^23): 4 x 8 137 / 1258 / 1733 / 104, 4 x 8 held
-// to 48 registers (more resident warps for a plan that waits on loads) 127 /
-// 1434 / 1676 / 142, 2 x 8 137 / 1252 / 1864 / 109, 8 x 8 at 48 registers 125 /
-// 1625 / 1692 / 137.  Not worth a trial: 1 x 16 150 / 1706 / 1797 / 114, 4 x 4
-// 151 / 1836 / 1809 / 105, 4 x 16 157 / 1883 / 1860 / 129, 40 registers.
+// GB300, call us (light C1 plan 2^24 rows / deep C2 2^26 / order-line C5 2^27 /
+// process_filter of six columns 2^23): 4 x 8 212 / 1436 / 2079 / 251, 4 x 8 held
+// to 48 registers (more resident warps for a plan that waits on loads) 210 / 1570
+// / 1967 / 297, 2 x 8 220 / 1419 / 2110 / 261, 8 x 8 at 48 registers 206 / 1767 /
+// 1995 / 291.  Not worth a trial: 1 x 16, 4 x 4 and 4 x 16 words, 40 registers.
 static const CompiledPlan::Shape kShapes[] = {{4, 8, 0}, {4, 8, 48}, {2, 8, 0}, {8, 8, 48}};
 static constexpr int kNumShapes = 4;
 // Small calls leave most of the chip idle, so a tile's latency counts: 8 x 4 has
